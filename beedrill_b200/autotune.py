@@ -47,8 +47,8 @@ BATCHED_SPACE = {
     "large_degree": [16, 32, 64, 128, 1024],
     "chunk_edges": [128, 256, 512, 1024],
     "pull_prefix": [8, 16, 32, 64],
-    "heavy_degree": [1024, 4096, 16384],
-    "heavy_chunk": [512, 2048, 8192],
+    "heavy_degree": [0, 64, 256, 1024, 4096],  # 0: the library's rule
+    "heavy_chunk": [0, 128, 512, 2048],
 }
 
 
@@ -118,7 +118,7 @@ def tune(scale=24, roots=64, seed=1024, order=bd.ORDER_HUB, log=None):
     single, s_score, s_table = coordinate_descent(
         SINGLE_SPACE, start_single, lambda p: score_single(g, rs, p), log)
     start_batched = {"block_size": 512, "alpha": 4, "large_degree": 32, "chunk_edges": 256,
-                     "pull_prefix": 16, "heavy_degree": 4096, "heavy_chunk": 2048}
+                     "pull_prefix": 16, "heavy_degree": 0, "heavy_chunk": 0}
     batched, b_score, b_table = coordinate_descent(
         BATCHED_SPACE, start_batched, lambda p: score_batched(g, rs[:64], p), log)
     g.close()

@@ -69,6 +69,7 @@ struct MsAcc {
     ull t_end;       // max over CTAs of their arrival time
     ull work;        // pull steps: next bitmap word to hand out
     ull lanes_or;    // lanes delivered in the step (the next frontier's lanes)
+    ull deferred;    // pull steps: chunks of long lists left for all warps
 };
 
 // State between steps: written first by the init kernel, then kept by every
@@ -83,10 +84,11 @@ struct MsState {
     long long t_last, push_steps, pull_steps;
     long long prev_ns, policy_overrides;
     ull active;                  // lanes the frontier about to be expanded holds
+    long long bars;              // grid barriers passed
 };
 
 struct MsCtrl {
-    ull bar;       // barrier arrivals; step s is complete at (s + 1) * CTAs
+    ull bar;       // barrier arrivals; barrier b is complete at (b + 1) * CTAs
     int error, pad0;
     ull t_start;   // min over CTAs of their start time
     MsState st;
@@ -120,12 +122,11 @@ struct MsParams {
     int force_dir;  // -1 rule, kPush, kPull
     const PolicyBlob *policy;  // null: the rule decides
     const uint32_t *perm;      // caller id -> traversal id (BD_ORDER_HUB), or null
-    // vertices whose pull scan is split into chunks over all warps
-    const uint32_t *heavy;           // [n_heavy]
-    const ull *heavy_cbase;          // [n_heavy + 1] chunk prefix sums
-    int64_t n_heavy;
-    int64_t heavy_deg;               // degree above which a vertex is heavy
-    uint32_t heavy_chunk;            // arcs per chunk
+    // pull scans longer than long_arcs: what is left after so many arcs goes to
+    // all warps in chunks of long_chunk arcs, listed in dq as {vertex, chunk}
+    uint2 *dq;         // null: no list of the graph is that long
+    int64_t long_arcs;
+    uint32_t long_chunk;
 };
 
 struct MsLocal {
@@ -487,13 +488,12 @@ __device__ void ms_push_step(const MsParams &p, const MsView &sv, MsWarpScratch 
     }
 }
 
-// pull: warp per 32 vertices; short lists per lane, long lists by the warp.
-// pull for heavy vertices: their lists are cut into chunks dealt to all
-// warps.  A chunk ORs the lanes it finds into the vertex's next frontier
-// word; the bits the atomic returns as new are the ones this chunk
-// delivered first, so their parents come from this chunk.
+// The part of a pull step that comes after ms_pull_step: the chunks of the long
+// lists it left, one chunk per warp at a time.  A chunk ORs the lanes it finds
+// into the vertex's next frontier word; the bits the atomic returns as new are
+// the ones this chunk delivered first, so their parents come from this chunk.
 template <int BLOCK>
-__device__ void ms_pull_heavy(const MsParams &p, const MsView &sv, MsLocal &loc)
+__device__ void ms_pull_long(const MsParams &p, const MsView &sv, MsLocal &loc)
 {
     const int lane = lane_id();
     const int warp = threadIdx.x >> 5;
@@ -502,24 +502,19 @@ __device__ void ms_pull_heavy(const MsParams &p, const MsView &sv, MsLocal &loc)
     const int cur = sv.step % 3, nxt = (sv.step + 1) % 3;
     MsAcc *acc = &p.ctrl->acc[sv.step % 3];
     const int new_level = sv.level + 1;
-    const long long total = p.n_heavy ? (long long)__ldg(&p.heavy_cbase[p.n_heavy]) : 0;
-    // chunks dealt round robin: the chunks of one heavy vertex run on
-    // different warps at once, and any of them may find the vertex's last
-    // missing lanes
+    const long long total = (long long)__ldcg(&acc->deferred);
+    // chunks dealt round robin: the chunks of one vertex run on different
+    // warps at once, and any of them may find the vertex's last missing lanes
     for (long long c = gw; c < total; c += nw) {
-        long long lo = 0, hi = p.n_heavy - 1;  // last i with heavy_cbase[i] <= c
-        while (lo < hi) {
-            const long long mid = (lo + hi + 1) >> 1;
-            if ((long long)__ldg(&p.heavy_cbase[mid]) <= c) { lo = mid; } else { hi = mid - 1; }
-        }
-        const uint32_t v = __ldg(&p.heavy[lo]);
+        const uint2 d = __ldcg(&p.dq[c]);
+        const uint32_t v = d.x;
         // lanes v lacks that the frontier holds (other chunks of v may have
         // delivered some already this step)
         const ull need = p.all & ~__ldcg(&p.reach[v]) & sv.active;
         if (!need) { continue; }
         const int64_t vb = __ldg(&p.off[v]), ve = __ldg(&p.off[v + 1]);
-        const int64_t b = vb + (c - (long long)__ldg(&p.heavy_cbase[lo])) * (int64_t)p.heavy_chunk;
-        const int64_t e = min(ve, b + (int64_t)p.heavy_chunk);
+        const int64_t b = vb + p.long_arcs + (int64_t)d.y * (int64_t)p.long_chunk;
+        const int64_t e = min(ve, b + (int64_t)p.long_chunk);
         ull have = 0;  // lanes this chunk found or saw others deliver
         for (int64_t base = b; base < e && (have & need) != need; base += 128) {
             uint32_t u[4];
@@ -578,6 +573,35 @@ __device__ __forceinline__ ull ms_next_chunk(ull *counter, long long nw, long lo
     return (ull)nw + __shfl_sync(kFullMask, x, 0);
 }
 
+// Warp-collective: lists the chunks of `rest` arcs of each lane with `has`.
+__device__ __forceinline__ void ms_defer(const MsParams &p, MsAcc *acc, bool has, uint32_t v,
+                                         int64_t rest)
+{
+    const unsigned k = has ? (unsigned)((rest + p.long_chunk - 1) / p.long_chunk) : 0u;
+    const unsigned incl = warp_incl_scan(k);
+    ull base = 0;
+    if (lane_id() == 31) { base = atomicAdd(&acc->deferred, (ull)incl); }
+    base = __shfl_sync(kFullMask, base, 31);
+    unsigned owners = __ballot_sync(kFullMask, k != 0);
+    while (owners) {
+        const int o = __ffs(owners) - 1;
+        owners &= owners - 1;
+        const unsigned n = __shfl_sync(kFullMask, k, o);
+        const ull at = base + __shfl_sync(kFullMask, incl, o) - n;
+        const uint32_t vo = __shfl_sync(kFullMask, v, o);
+        for (unsigned i = lane_id(); i < n; i += 32) { p.dq[at + i] = make_uint2(vo, i); }
+    }
+}
+
+// pull: warp per 32 vertices; a lane scans the first `prefix` arcs of its own
+// vertex, the warp goes on with the lists that still lack lanes, one after
+// another, up to long_arcs arcs of each; what is left of longer lists is put on
+// dq for all warps (ms_pull_long).  Leaving no long list to one warp is what
+// bounds the step: a hub numbering puts 32 vertices of the highest degrees into
+// one warp's word, and a lane of the batch whose frontier is still small keeps
+// every scan from ending early.  With only lists above 4096 arcs dealt out, the
+// first pull of 64 roots at scale 20 took 100 us or 1,170 us, by whether the
+// batch had such a lane.
 template <int BLOCK>
 __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
 {
@@ -625,13 +649,6 @@ __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
                 if (need) {
                     beg = __ldg(&p.off[v]);
                     end = __ldg(&p.off[v + 1]);
-                    if (end - beg > p.heavy_deg) {
-                        // scanned in chunks by ms_pull_heavy
-                        need = 0;
-                        beg = end = 0;
-                    }
-                }
-                if (need) {
                     cnt = cnt0 = __ldcg(&p.drec_cnt[v]);
                     const int64_t lim = min(end, beg + (int64_t)p.prefix);
                     int64_t k = beg;
@@ -657,12 +674,13 @@ __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
                     next = (got == need) ? end : min(k, lim);
                 }
             }
-            unsigned pending = __ballot_sync(kFullMask, need != 0 && got != need && next < end);
+            const int64_t stop = p.dq ? min(end, beg + p.long_arcs) : end;
+            unsigned pending = __ballot_sync(kFullMask, need != 0 && got != need && next < stop);
             while (pending) {
                 const int owner = __ffs(pending) - 1;
                 pending &= pending - 1;
                 const int64_t b = __shfl_sync(kFullMask, next, owner);
-                const int64_t e = __shfl_sync(kFullMask, end, owner);
+                const int64_t e = __shfl_sync(kFullMask, stop, owner);
                 const ull nd = __shfl_sync(kFullMask, need, owner);
                 ull have = __shfl_sync(kFullMask, got, owner);
                 const uint32_t vo = __shfl_sync(kFullMask, v, owner);
@@ -702,13 +720,17 @@ __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
                 }
             }
             if (cnt != cnt0) { p.drec_cnt[v] = cnt; }
+            if (p.dq) {
+                const bool more = need != 0 && got != need && stop < end;
+                if (__any_sync(kFullMask, more)) { ms_defer(p, acc, more, v, end - stop); }
+            }
             const bool gained = got != 0;
             const bool completed = gained && ((s | got) & p.all) == p.all;
             const unsigned cm = __ballot_sync(kFullMask, completed);
             if (lane == 0 && cm) { atomicOr(&p.done[w], cm); }
             if (gained) {
-                // v is this lane's alone in a pull step (heavy vertices are
-                // left to ms_pull_heavy), so plain stores
+                // v is this lane's alone until the barrier before
+                // ms_pull_long, so plain stores
                 p.F[nxt][v] = got;
                 p.reach[v] = s | got;
                 loc.lanes += __popcll(got);
@@ -720,6 +742,25 @@ __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
     }
 }
 
+// Grid barrier: arrival (one release-add per CTA) and acquire polling until
+// every CTA has arrived.  Bounded by p.spin_limit polls.  Thread 0 of each CTA;
+// b is the number of barriers passed before.
+__device__ __forceinline__ bool ms_arrive_wait(const MsParams &p, long long b)
+{
+    MsCtrl *c = p.ctrl;
+    red_release_add64(&c->bar, 1ull);
+    const ull target = (ull)(b + 1) * p.expected_ctas;
+    long long it = 0;
+    while (ld_acquire64(&c->bar) < target) {
+        if (++it > p.spin_limit) {
+            atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
+            return false;
+        }
+        __nanosleep(32);
+    }
+    return true;
+}
+
 template <int BLOCK>
 struct MsShared {
     MsWarpScratch warp[BLOCK / 32];
@@ -727,6 +768,7 @@ struct MsShared {
     MsState st;     // this CTA's copy of the state
     PolicyBlob pol; // the learned policy's weights, staged once
     int rule_dir;
+    bool listed;    // pull step: all chunks of long lists are on dq
 };
 
 // The rule: pull once the frontier's edges are a sizeable share of the edges
@@ -830,22 +872,12 @@ __device__ void ms_end_step(const MsParams &p, const MsView &sv, MsShared<BLOCK>
         if (blockIdx.x == 0) {
             MsAcc *z = &c->acc[(s + 1) % 3];
             z->vertices = z->degsum = z->lanes = z->small_cnt = z->large_packed = 0;
-            z->done_degsum = z->t_end = z->work = z->lanes_or = 0;
+            z->done_degsum = z->t_end = z->work = z->lanes_or = z->deferred = 0;
         }
         atomicMax(&acc->t_end, (ull)globaltimer());
-        red_release_add64(&c->bar, 1ull);
-        const ull target = (ull)(s + 1) * p.expected_ctas;
-        long long it = 0;
-        bool ok = true;
-        while (ld_acquire64(&c->bar) < target) {
-            if (++it > p.spin_limit) {
-                atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
-                ok = false;
-                break;
-            }
-            __nanosleep(32);
-        }
         MsState &st = sh.st;
+        const bool ok = ms_arrive_wait(p, st.bars);
+        st.bars += 1;
         if (ok && __ldcg(&c->error) == 0) {
             MsAcc a;
             a.vertices = __ldcg(&acc->vertices);
@@ -902,8 +934,19 @@ __global__ void __launch_bounds__(BLOCK, MINB) msbfs_kernel(MsParams p)
         if (sv.dir == kPush) {
             ms_push_step<BLOCK>(p, sv, sh.warp[threadIdx.x >> 5], loc);
         } else {
-            ms_pull_heavy<BLOCK>(p, sv, loc);
             ms_pull_step<BLOCK>(p, sv, loc);
+            if (p.dq) {
+                // every CTA's part of the lists is scanned and its chunks are
+                // listed (after a timeout they may not all be: none is read, and
+                // the end of the step sees the error)
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    sh.listed = ms_arrive_wait(p, sh.st.bars);
+                    sh.st.bars += 1;
+                }
+                __syncthreads();
+                if (sh.listed) { ms_pull_long<BLOCK>(p, sv, loc); }
+            }
         }
         ms_end_step<BLOCK>(p, sv, sh, loc);
     }
@@ -1296,6 +1339,19 @@ __global__ void __launch_bounds__(kMatThreads) ms_materialize_kernel(MsOutParams
     }
 }
 
+__global__ void ms_long_chunks_kernel(const int64_t *off, int64_t n, int64_t long_arcs,
+                                      uint32_t long_chunk, ull *chunks)
+{
+    ull c = 0;
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t rest = off[v + 1] - off[v] - long_arcs;
+        if (rest > 0) { c += (ull)((rest + long_chunk - 1) / long_chunk); }
+    }
+    c = warp_sum(c);
+    if (lane_id() == 0 && c) { atomicAdd(chunks, c); }
+}
+
 using MsKernel = void (*)(MsParams);
 
 int ms_grid_for(int64_t items)
@@ -1339,9 +1395,7 @@ struct bd_msbfs {
     std::vector<int64_t> sources;  // roots of the last run
     bool ran = false;
     PolicyBlob *policy = nullptr;  // device copy, or null
-    uint32_t *heavy = nullptr;
-    ull *heavy_cbase = nullptr;
-    int64_t n_heavy = 0;
+    uint2 *dq = nullptr;  // chunks of long pull scans, or null: no list is that long
     cudaGraphExec_t graph = nullptr;
     int graph_count = -1;
     bool graph_ok = true;
@@ -1402,11 +1456,9 @@ MsParams ms_params(bd_msbfs *b, int group, int count)
     p.expected_ctas = (unsigned)b->grid;
     p.force_dir = b->opts.force_dir;
     p.policy = b->policy;
-    p.heavy = b->heavy;
-    p.heavy_cbase = b->heavy_cbase;
-    p.n_heavy = b->n_heavy;
-    p.heavy_deg = b->opts.heavy_degree;
-    p.heavy_chunk = (uint32_t)b->opts.heavy_chunk;
+    p.dq = b->dq;
+    p.long_arcs = b->opts.heavy_degree;
+    p.long_chunk = (uint32_t)b->opts.heavy_chunk;
     return p;
 }
 
@@ -1540,8 +1592,7 @@ void ms_free(bd_msbfs *b)
     cudaFree(b->d_sources);
     cudaFree(b->d_counts);
     cudaFree(b->policy);
-    cudaFree(b->heavy);
-    cudaFree(b->heavy_cbase);
+    cudaFree(b->dq);
     cudaFree(b->out_depth);
     cudaFree(b->out_parent);
     cudaFree(b->xbuf);
@@ -1549,6 +1600,21 @@ void ms_free(bd_msbfs *b)
     if (b->ev1) { cudaEventDestroy(b->ev1); }
     if (b->stream) { cudaStreamDestroy(b->stream); }
     delete b;
+}
+
+// Chunks of the arcs past opts.heavy_degree over all lists of the traversal CSR
+// (counted in the handle's d_counts, which no run uses yet).
+bd_status ms_long_chunks(bd_msbfs *b, unsigned long long *chunks)
+{
+    BD_CUDA(cudaMemsetAsync(b->d_counts, 0, sizeof(unsigned long long), b->stream));
+    ms_long_chunks_kernel<<<ms_grid_for(b->g->n), 256, 0, b->stream>>>(
+        traversal_off(b->g), b->g->n, b->opts.heavy_degree, (uint32_t)b->opts.heavy_chunk,
+        b->d_counts);
+    BD_CUDA(cudaGetLastError());
+    BD_CUDA(cudaMemcpyAsync(chunks, b->d_counts, sizeof(*chunks), cudaMemcpyDeviceToHost,
+                            b->stream));
+    BD_CUDA(cudaStreamSynchronize(b->stream));
+    return BD_OK;
 }
 
 bd_status ms_check_root(bd_msbfs *b, int32_t root_index)
@@ -1629,8 +1695,6 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
     if (o.large_degree > (1 << 20)) { return BD_ERR_INVALID; }
     if (o.chunk_edges <= 0) { o.chunk_edges = 256; }
     if (o.pull_prefix <= 0) { o.pull_prefix = 16; }
-    if (o.heavy_degree <= 0) { o.heavy_degree = 4096; }
-    if (o.heavy_chunk <= 0) { o.heavy_chunk = 2048; }
     if (o.spin_limit <= 0) { o.spin_limit = kMsDefaultSpin; }
     if (o.materialize < 0 || o.materialize > 1 || o.min_parent < 0 || o.min_parent > 1) {
         return BD_ERR_INVALID;
@@ -1698,30 +1762,34 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
         return fail(BD_ERR_CUDA);
     }
     b->grid = per_sm * sms;
-    // heavy vertices and their chunk prefix sums (host, once per handle)
+    // Where a pull scan leaves a list to all warps (0 = this rule).  A warp takes
+    // a word of 32 vertices, so up to 32 x heavy_degree arcs one after another;
+    // that should not exceed what the average warp scans in a full pull, arcs /
+    // warps.  64 roots on the hub layout, traversal ms by heavy_degree:
+    //   scale 16 (rule 32)    32: 0.18   64: 0.20   256: 0.28   4096: 0.73
+    //   scale 20 (rule 218)   96: 0.48   192: 0.46  512: 0.53   4096: 1.37
+    //   scale 22 (rule 886)  256: 1.14   512: 1.13  1024: 1.19  4096: 1.40
+    //   scale 24 (rule 3430) 512: 3.66  1024: 3.61  4096: 3.56
+    // (scales 20 and 22: batches with a lane whose frontier is still small).
+    // Shorter lists than 32 arcs are not worth a chunk; above 4096 arcs even the
+    // largest graphs gain by dealing them out.
+    const int64_t warps = (int64_t)b->grid * (b->block / 32);
+    if (b->opts.heavy_degree <= 0) {
+        b->opts.heavy_degree =
+            (int32_t)std::min<int64_t>(4096, std::max<int64_t>(32, g->arcs / (32 * warps)));
+    }
+    // chunks of a few such lengths: scale 16 128 arcs 0.18, 512 0.20; scale 20
+    // 128: 0.40, 512: 0.39
+    if (b->opts.heavy_chunk <= 0) {
+        b->opts.heavy_chunk = std::min(2048, std::max(128, 4 * b->opts.heavy_degree));
+    }
+    b->opts.pull_prefix = std::min(b->opts.pull_prefix, b->opts.heavy_degree);
+    // room for every chunk a pull step can leave to ms_pull_long
     {
-        std::vector<int64_t> off(n + 1);
-        if (cudaMemcpy(off.data(), traversal_off(g), sizeof(int64_t) * (n + 1),
-                       cudaMemcpyDeviceToHost) !=
-            cudaSuccess) {
-            return fail(BD_ERR_CUDA);
-        }
-        std::vector<uint32_t> hv;
-        std::vector<ull> hc(1, 0);
-        for (int64_t v = 0; v < n; ++v) {
-            const int64_t d = off[v + 1] - off[v];
-            if (d > o.heavy_degree) {
-                hv.push_back((uint32_t)v);
-                hc.push_back(hc.back() + (ull)((d + o.heavy_chunk - 1) / o.heavy_chunk));
-            }
-        }
-        b->n_heavy = (int64_t)hv.size();
-        if (cudaMalloc(&b->heavy, sizeof(uint32_t) * std::max<size_t>(hv.size(), 1)) != cudaSuccess ||
-            cudaMalloc(&b->heavy_cbase, sizeof(ull) * hc.size()) != cudaSuccess ||
-            (!hv.empty() && cudaMemcpy(b->heavy, hv.data(), sizeof(uint32_t) * hv.size(),
-                                       cudaMemcpyHostToDevice) != cudaSuccess) ||
-            cudaMemcpy(b->heavy_cbase, hc.data(), sizeof(ull) * hc.size(), cudaMemcpyHostToDevice) !=
-                cudaSuccess) {
+        ull chunks = 0;
+        const bd_status st = ms_long_chunks(b, &chunks);
+        if (st != BD_OK) { return fail(st); }
+        if (chunks && cudaMalloc(&b->dq, sizeof(uint2) * chunks) != cudaSuccess) {
             return fail(BD_ERR_OOM);
         }
     }

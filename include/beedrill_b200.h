@@ -289,9 +289,10 @@ typedef struct bd_msbfs_opts {
     int32_t use_graph;     /* 1 (default via bd_msbfs_default_opts): replay the
                               groups of a call as one captured CUDA graph       */
     int64_t spin_limit;    /* grid-barrier poll bound; 0 = default (~2 s)       */
-    int32_t heavy_degree;  /* pull: lists longer than this are cut into chunks
-                              shared by all warps; 0 = default (4096)           */
-    int32_t heavy_chunk;   /* arcs per such chunk; 0 = default (2048)           */
+    int32_t heavy_degree;  /* pull: a scan still unfinished after so many arcs
+                              leaves the rest in chunks to all warps; 0 =
+                              default (32 to 4096, by the size of the graph)    */
+    int32_t heavy_chunk;   /* arcs per such chunk; 0 = default (128 to 2048)    */
     int32_t materialize;   /* 1: every run ends with each root's int32 depths
                               and int64 parents (caller ids, the reference's
                               encoding) in device memory owned by the handle,
