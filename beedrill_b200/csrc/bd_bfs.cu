@@ -45,11 +45,11 @@ struct StepView {
     int level;
     int vis_cur;
     int q_cur;
-    int step;
     int bu_sparse;
     long long f_small;
     long long f_large;
     long long f_chunks;
+    long long barrier;
 };
 
 __device__ __forceinline__ StepView view_of(const LevelState &s)
@@ -60,7 +60,7 @@ __device__ __forceinline__ StepView view_of(const LevelState &s)
     v.level = s.level;
     v.vis_cur = s.vis_cur;
     v.q_cur = s.q_cur;
-    v.step = s.step;
+    v.barrier = s.barrier;
     v.f_small = s.f_small;
     v.f_large = s.f_large;
     v.f_chunks = s.f_chunks;
@@ -155,6 +155,12 @@ __device__ __forceinline__ int64_t degree_of(const BfsParams &p, uint32_t v)
     return __ldg(&p.off[v + 1]) - __ldg(&p.off[v]);
 }
 
+// The warps that share a step (the grid's, or CTA 0's) and its counters.
+struct Team {
+    long long gw, nw;  // this warp among nw
+    Acc *acc;
+};
+
 constexpr int kILP = 4;
 
 // Top-down claims of a batch of kILP neighbours per lane (hybrid_bfs.cc:83-96):
@@ -216,27 +222,55 @@ struct WarpScratch {
     int64_t beg[32];
 };
 
+// Bounds of the levels CTA 0 runs alone (solo_run).
+template <int BLOCK>
+constexpr int kSoloCap = BLOCK / 8 * 5;
+template <int BLOCK>
+constexpr long long kSoloArcs = 5 * BLOCK;
+template <int BLOCK>
+constexpr long long kSoloBu = 8 * BLOCK;
+template <int BLOCK>
+constexpr long long kSoloBuArcs = 64 * BLOCK;
+
+// Two queues of vertices: id, low word of the list start, and its high 16 bits
+// with the degree (65535: that or more), which becomes the position of the list's
+// first arc when the level is run (below 2^16, as kSoloArcs is).
+template <int BLOCK>
+struct SoloQueues {
+    uint32_t v[2][kSoloCap<BLOCK>];
+    uint32_t lo[2][kSoloCap<BLOCK>];
+    uint32_t hi[2][kSoloCap<BLOCK>];
+};
+
 template <int BLOCK>
 struct SharedState {
-    WarpScratch warp[BLOCK / 32];
+    union {
+        WarpScratch warp[BLOCK / 32];   // the grid's top-down steps
+        SoloQueues<BLOCK> queues;       // CTA 0's narrow levels
+    };
     unsigned long long red_found[BLOCK / 32];
     unsigned long long red_deg[BLOCK / 32];
     LevelState st;       // this CTA's copy of the traversal state
     PolicyBlob pol;      // the learned policy's weights, staged once
     int rule_dir;
+    int consult;         // the learned policy decides the next step
+    // CTA 0's narrow levels
+    BfsParams par;       // the launch's parameters, for code that is not inlined
+    Acc acc;             // counters (queue entries past the shared queue too)
+    unsigned queued;     // entries of the queue being filled
+    unsigned warp_sum[BLOCK / 32];
 };
 
 template <int BLOCK>
-__device__ void td_step(const BfsParams &p, const StepView &sv, SharedState<BLOCK> &sh,
-                        Local &loc)
+__device__ void td_step(const BfsParams &p, const StepView &sv, const Team &team,
+                        SharedState<BLOCK> &sh, Local &loc)
 {
     const int lane = lane_id();
     const int warp = threadIdx.x >> 5;
-    const long long gw = (long long)blockIdx.x * (BLOCK / 32) + warp;
-    const long long nw = (long long)gridDim.x * (BLOCK / 32);
+    const long long gw = team.gw, nw = team.nw;
     const int qin = sv.q_cur, qout = sv.q_cur ^ 1;
     uint32_t *vis = p.vis[sv.vis_cur];
-    Acc *acc = &p.ctrl->acc[sv.step % 3];
+    Acc *acc = team.acc;
     const int new_level = sv.level + 1;
 
     // Phase A: chunks of large-degree frontier vertices.  Warp gw takes a
@@ -326,17 +360,15 @@ __device__ void td_step(const BfsParams &p, const StepView &sv, SharedState<BLOC
 // 32 arcs per ballot (warp-ballot early exit).  Reads only the frozen bitmap
 // vis[cur]; writes whole words of vis[cur^1].
 template <int BLOCK, int K>
-__device__ void bu_step(const BfsParams &p, const StepView &sv, Local &loc)
+__device__ void bu_step(const BfsParams &p, const StepView &sv, const Team &team, Local &loc)
 {
     constexpr int P = K >= 4 ? 2 : 4;
     const int lane = lane_id();
-    const int warp = threadIdx.x >> 5;
-    const long long gw = (long long)blockIdx.x * (BLOCK / 32) + warp;
-    const long long nw = (long long)gridDim.x * (BLOCK / 32);
+    const long long gw = team.gw, nw = team.nw;
     const uint32_t *vin = p.vis[sv.vis_cur];
     uint32_t *vout = p.vis[sv.vis_cur ^ 1];
     const int qout = sv.q_cur ^ 1;
-    Acc *acc = &p.ctrl->acc[sv.step % 3];
+    Acc *acc = team.acc;
     const int new_level = sv.level + 1;
 
     // Warp gw owns groups gw, gw + nw, gw + 2 nw, ... of K words.  It loads
@@ -363,64 +395,69 @@ __device__ void bu_step(const BfsParams &p, const StepView &sv, Local &loc)
             uint32_t word[K];
 #pragma unroll
             for (int k = 0; k < K; ++k) { word[k] = __shfl_sync(kFull, mw, g * K + k); }
-            uint32_t v[K], par[K];
-            bool found[K], unv[K];
-            int64_t beg[K], end[K], next[K];
+            // Per word only the list start, its length and the parent are kept
+            // (open / fnd hold the flags, one bit per word), so that K = 4 fits
+            // the 64 registers of a full SM.
+            const uint32_t v0 = (uint32_t)(w0 * 32 + lane);
+            unsigned open = 0, fnd = 0;
+            uint32_t par[K], len[K];  // length: 2^32 - 1 stands for that or more
+            int64_t beg[K];
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                v[k] = (uint32_t)((w0 + k) * 32 + lane);
-                unv[k] = !((word[k] >> lane) & 1u);
-                found[k] = false;
-                par[k] = 0;
-                beg[k] = end[k] = next[k] = 0;
-                if (unv[k]) {
-                    beg[k] = __ldg(&p.off[v[k]]);
-                    end[k] = __ldg(&p.off[v[k] + 1]);
+                par[k] = len[k] = 0;
+                beg[k] = 0;
+                if (!((word[k] >> lane) & 1u)) {
+                    open |= 1u << k;
+                    beg[k] = __ldg(&p.off[v0 + 32 * k]);
+                    len[k] = (uint32_t)min(__ldg(&p.off[v0 + 32 * k + 1]) - beg[k], (int64_t)kFull);
                 }
             }
             // per-lane scan of the first bu_prefix arcs, P arcs per word per round
-            for (int r = 0; r < p.bu_prefix; r += P) {
-                uint32_t x[K][P];
-                bool in[K][P];
+            const uint32_t lim = (uint32_t)(p.bu_prefix + P - 1) / P * P;
+            for (uint32_t r = 0; r < lim; r += P) {
+                uint32_t x[K][P], hit[K][P];
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
 #pragma unroll
                     for (int j = 0; j < P; ++j) {
-                        const int64_t e = beg[k] + r + j;
-                        in[k][j] = unv[k] && !found[k] && e < end[k];
-                        x[k][j] = in[k][j] ? __ldg(&p.adj[e]) : 0u;
+                        x[k][j] = (open >> k) & 1u && r + j < len[k] ? __ldg(&p.adj[beg[k] + r + j]) : 0u;
                     }
                 }
-                uint32_t bits[K][P];
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
 #pragma unroll
-                    for (int j = 0; j < P; ++j) { bits[k][j] = in[k][j] ? ld_bits(&vin[x[k][j] >> 5]) : 0u; }
+                    for (int j = 0; j < P; ++j) {
+                        hit[k][j] = (open >> k) & 1u && r + j < len[k]
+                                        ? (ld_bits(&vin[x[k][j] >> 5]) >> (x[k][j] & 31)) & 1u
+                                        : 0u;
+                    }
                 }
                 bool more = false;
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
 #pragma unroll
                     for (int j = 0; j < P; ++j) {
-                        if (in[k][j] && !found[k] && ((bits[k][j] >> (x[k][j] & 31)) & 1u)) {
-                            found[k] = true;
+                        if (hit[k][j] && (open >> k) & 1u) {
+                            fnd |= 1u << k;
+                            open &= ~(1u << k);
                             par[k] = x[k][j];
                         }
                     }
-                    more |= unv[k] && !found[k] && beg[k] + r + P < end[k];
+                    more |= (open >> k) & 1u && r + P < len[k];
                 }
                 if (!__any_sync(kFull, more)) { break; }
             }
+            bool found[K];
+            uint32_t v[K];
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const int64_t lim = min(end[k], beg[k] + (int64_t)((p.bu_prefix + P - 1) / P * P));
-                next[k] = found[k] ? end[k] : lim;
-                unsigned pending = __ballot_sync(kFull, unv[k] && !found[k] && next[k] < end[k]);
+                v[k] = v0 + 32 * k;
+                unsigned pending = __ballot_sync(kFull, (open >> k) & 1u && len[k] > lim);
                 while (pending) {
                     const int owner = __ffs(pending) - 1;
                     pending &= pending - 1;
-                    const int64_t b = __shfl_sync(kFull, next[k], owner);
-                    const int64_t e = __shfl_sync(kFull, end[k], owner);
+                    const int64_t b = __shfl_sync(kFull, beg[k], owner) + lim;
+                    const int64_t e = __ldg(&p.off[__shfl_sync(kFull, v[k], owner) + 1]);
                     for (int64_t base = b; base < e; base += 32) {
                         const int64_t kk = base + lane;
                         bool hit = false;
@@ -433,13 +470,14 @@ __device__ void bu_step(const BfsParams &p, const StepView &sv, Local &loc)
                         if (hm) {
                             const uint32_t hx = __shfl_sync(kFull, xx, __ffs(hm) - 1);
                             if (lane == owner) {
-                                found[k] = true;
+                                fnd |= 1u << k;
                                 par[k] = hx;
                             }
                             break;
                         }
                     }
                 }
+                found[k] = (fnd >> k) & 1u;
                 const unsigned fm = __ballot_sync(kFull, found[k]);
                 if (lane == 0 && w0 + k < p.words) { vout[w0 + k] = word[k] | fm; }
                 if (found[k]) {
@@ -449,7 +487,9 @@ __device__ void bu_step(const BfsParams &p, const StepView &sv, Local &loc)
             }
             int64_t deg[K];
 #pragma unroll
-            for (int k = 0; k < K; ++k) { deg[k] = end[k] - beg[k]; }
+            for (int k = 0; k < K; ++k) {
+                deg[k] = len[k] == kFull ? degree_of(p, v[k]) : (int64_t)len[k];
+            }
             warp_append_k<K>(p, acc, qout, found, v, deg, loc);
         }
     }
@@ -465,17 +505,15 @@ __device__ void bu_step(const BfsParams &p, const StepView &sv, Local &loc)
 constexpr int64_t kLongList = 256;
 
 template <int BLOCK>
-__device__ void bu_step_lanes(const BfsParams &p, const StepView &sv, Local &loc)
+__device__ void bu_step_lanes(const BfsParams &p, const StepView &sv, const Team &team, Local &loc)
 {
     constexpr int P = 4;
     const int lane = lane_id();
-    const int warp = threadIdx.x >> 5;
-    const long long gw = (long long)blockIdx.x * (BLOCK / 32) + warp;
-    const long long nw = (long long)gridDim.x * (BLOCK / 32);
+    const long long gw = team.gw, nw = team.nw;
     const uint32_t *vin = p.vis[sv.vis_cur];
     uint32_t *vout = p.vis[sv.vis_cur ^ 1];
     const int qout = sv.q_cur ^ 1;
-    Acc *acc = &p.ctrl->acc[sv.step % 3];
+    Acc *acc = team.acc;
     const int new_level = sv.level + 1;
 
     for (long long base = gw * 32; base < p.words; base += nw * 32) {
@@ -611,7 +649,10 @@ __device__ void bu_step_lanes(const BfsParams &p, const StepView &sv, Local &loc
 __device__ int beamer_choose(LevelState &c, const BfsParams &p, bool commit)
 {
     if (c.in_bu) { return kDirBU; }
-    if (c.scout > c.etc / p.alpha) {
+    // scout > etc / alpha, without the division where the product fits
+    const bool pull = c.etc >= 0 && ((c.scout | p.alpha) >> 31) == 0 ? c.scout * p.alpha > c.etc
+                                                                     : c.scout > c.etc / p.alpha;
+    if (pull) {
         if (commit) {
             c.in_bu = 1;
             c.awake = c.f_count;  // queue_.combined_size()
@@ -678,23 +719,29 @@ __device__ int apply_policy(LevelState &c, const PolicyBlob *w, int rule, float 
     return d;
 }
 
-// Picks c.dir for the next step: thread 0 applies the rule, warp 0 runs the
-// policy network from w (shared or global memory) where it applies.  Called
-// by every thread of the block.
-template <typename Shared>
-__device__ void decide_next(LevelState &c, const BfsParams &p, const PolicyBlob *w, Shared &sh)
+// Picks c.dir for the next step: thread 0 applies the rule (in the branch that
+// advanced the state), warp 0 runs the policy network where it applies.
+__device__ __forceinline__ void decide_rule(LevelState &c, const BfsParams &p, int &rule_dir,
+                                            int &consult)
 {
-    if (threadIdx.x == 0) { sh.rule_dir = rule_direction(c, p); }
-    __syncthreads();
-    if (!policy_applies(c, p)) {
-        if (threadIdx.x == 0) { c.dir = sh.rule_dir; }
-        return;
-    }
+    consult = policy_applies(c, p);
+    rule_dir = rule_direction(c, p);
+    if (!consult) { c.dir = rule_dir; }
+}
+
+// After decide_rule and a block barrier; every thread of the block.  Ends with
+// the decision visible to the block.
+template <typename Shared>
+__device__ __forceinline__ void decide_policy(const BfsParams &p, Shared &sh)
+{
+    if (!sh.consult) { return; }
     if (threadIdx.x < 32) {
-        const float gap = policy_gap_warp(w, c.f_count, c.f_degsum, 2 * p.m - c.visited_degsum,
+        LevelState &c = sh.st;
+        const float gap = policy_gap_warp(&sh.pol, c.f_count, c.f_degsum, 2 * p.m - c.visited_degsum,
                                           c.level, p.n, p.m, c.prev_dir, c.prev_ns);
-        if (threadIdx.x == 0) { c.dir = apply_policy(c, w, sh.rule_dir, gap); }
+        if (threadIdx.x == 0) { c.dir = apply_policy(c, &sh.pol, sh.rule_dir, gap); }
     }
+    __syncthreads();
 }
 
 // Advances the state over the step that just ended, from that step's
@@ -728,17 +775,12 @@ __device__ void advance(LevelState &c, const BfsParams &p, const Acc &a, long lo
     c.step += 1;
 }
 
-// The end of a step: block reduction of the counters, arrival at the grid
-// barrier (one release-add per CTA), acquire polling until every CTA has
-// arrived, then every CTA advances its copy of the state from the step's
-// counters and decides the next direction.  Every wait is bounded by
-// p.spin_limit polls; running out sets ctrl->error = BD_ERR_TIMEOUT and ends
-// this CTA's loop.
+// Sums the block's step counters into acc->found / degsum (any memory) from
+// thread 0.  Ends after a block barrier; the sums are thread 0's.
 template <int BLOCK>
-__device__ void end_step(const BfsParams &p, const StepView &sv, SharedState<BLOCK> &sh,
-                         Local &loc)
+__device__ __forceinline__ void block_totals(SharedState<BLOCK> &sh, Local &loc,
+                                             unsigned long long &tf, unsigned long long &td)
 {
-    Ctrl *c = p.ctrl;
     const int lane = lane_id();
     const int warp = threadIdx.x >> 5;
     const unsigned long long f = warp_sum(loc.found);
@@ -750,85 +792,446 @@ __device__ void end_step(const BfsParams &p, const StepView &sv, SharedState<BLO
     loc.found = 0;
     loc.degsum = 0;
     __syncthreads();
+    tf = td = 0;
     if (threadIdx.x == 0) {
-        unsigned long long tf = 0, td = 0;
+#pragma unroll
         for (int i = 0; i < BLOCK / 32; ++i) {
             tf += sh.red_found[i];
             td += sh.red_deg[i];
         }
-        const int s = sv.step;
-        Acc *acc = &c->acc[s % 3];
+    }
+}
+
+// The step record of the step that just ended (before advance).
+__device__ __forceinline__ void record_step(const BfsParams &p, const LevelState &st,
+                                            long long found, long long t_end)
+{
+    if (st.step >= p.rec_cap) { return; }
+    bd_step r;
+    r.dir = st.dir;
+    r.level = st.level;
+    r.frontier = st.f_count;
+    r.frontier_edges = st.f_degsum;
+    r.unexplored_edges = 2 * p.m - st.visited_degsum;
+    r.found = found;
+    r.ns = t_end - st.t_last;
+    p.rec[st.step] = r;
+}
+
+// Grid barrier number b: arrival (one release-add) and polling until every CTA
+// has arrived, at most p.spin_limit polls; running out sets
+// ctrl->error = BD_ERR_TIMEOUT.  Thread 0 of each CTA.  False after an error.
+__device__ __forceinline__ bool arrive_wait(const BfsParams &p, long long b, bool solo)
+{
+    Ctrl *c = p.ctrl;
+    red_release_add64(&c->bar, 1ull);
+    const unsigned long long target = (unsigned long long)(b + 1) * p.expected_ctas;
+    long long it = 0;
+    // During CTA 0's narrow levels the others poll relaxed: an acquire load
+    // empties the SM's L1, and CTA 0 shares its SM (its reads, spilled registers
+    // among them, then went to L2: 4.1 us a level instead of 2.6).  At the end of
+    // a grid step the waits are short, and a poll that is itself the acquire
+    // saves a round trip (0.4 us a level).
+    while (solo && ld_relaxed64(&c->bar) < target) {
+        if (++it > p.spin_limit) {
+            atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
+            return false;
+        }
+        __nanosleep(64);
+    }
+    while (ld_acquire64(&c->bar) < target) {
+        if (++it > p.spin_limit) {
+            atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
+            return false;
+        }
+        __nanosleep(32);
+    }
+    return __ldcg(&c->error) == 0;
+}
+
+// CTA 0's part of a barrier's counter ring: the next barrier's slot.
+__device__ __forceinline__ void clear_next_acc(Ctrl *c, long long b)
+{
+    Acc *z = &c->acc[(b + 1) % 3];
+    z->found = z->degsum = z->small_cnt = z->large_packed = z->t_end = 0;
+}
+
+// The end of a step: block reduction of the counters, the grid barrier, then
+// every CTA advances its copy of the state from the step's counters and decides
+// the next direction.  A timeout ends this CTA's loop.
+template <int BLOCK>
+__device__ void end_step(const BfsParams &p, const StepView &sv, SharedState<BLOCK> &sh,
+                         Local &loc)
+{
+    Ctrl *c = p.ctrl;
+    unsigned long long tf, td;
+    block_totals<BLOCK>(sh, loc, tf, td);
+    if (threadIdx.x == 0) {
+        Acc *acc = &c->acc[sv.barrier % 3];
         if (tf) { atomicAdd(&acc->found, tf); }
         if (td) { atomicAdd(&acc->degsum, td); }
-        if (blockIdx.x == 0) {
-            Acc *z = &c->acc[(s + 1) % 3];
-            z->found = z->degsum = z->small_cnt = z->large_packed = z->t_end = 0;
-        }
+        if (blockIdx.x == 0) { clear_next_acc(c, sv.barrier); }
         atomicMax(&acc->t_end, (unsigned long long)globaltimer());
-        red_release_add64(&c->bar, 1ull);
-        const unsigned long long target = (unsigned long long)(s + 1) * p.expected_ctas;
-        long long it = 0;
-        bool ok = true;
-        while (ld_acquire64(&c->bar) < target) {
-            if (++it > p.spin_limit) {
-                atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
-                ok = false;
-                break;
-            }
-            __nanosleep(32);
-        }
-        if (ok && __ldcg(&c->error) == 0) {
+        LevelState &st = sh.st;
+        if (arrive_wait(p, sv.barrier, false)) {
             Acc a;
             a.found = __ldcg(&acc->found);
             a.degsum = __ldcg(&acc->degsum);
             a.small_cnt = __ldcg(&acc->small_cnt);
             a.large_packed = __ldcg(&acc->large_packed);
             const long long t_end = (long long)__ldcg(&acc->t_end);
-            LevelState &st = sh.st;
-            if (s == 0) { st.t_last = (long long)__ldcg(&c->t_start); }
-            if (blockIdx.x == 0 && s < p.rec_cap) {
-                bd_step r;
-                r.dir = st.dir;
-                r.level = st.level;
-                r.frontier = st.f_count;
-                r.frontier_edges = st.f_degsum;
-                r.unexplored_edges = 2 * p.m - st.visited_degsum;
-                r.found = (long long)a.found;
-                r.ns = t_end - st.t_last;
-                p.rec[s] = r;
-            }
+            if (blockIdx.x == 0) { record_step(p, st, (long long)a.found, t_end); }
             advance(st, p, a, t_end);
         } else {
-            sh.st.f_count = 0;  // leave the loop
+            st.f_count = 0;  // leave the loop
         }
+        st.barrier += 1;
+        decide_rule(st, p, sh.rule_dir, sh.consult);
     }
     __syncthreads();
-    decide_next(sh.st, p, &sh.pol, sh);
-    __syncthreads();
+    decide_policy(p, sh);
 }
 
 // K bitmap words per warp step: 1, 2, 4 (warp-shared words) or 32 (one word
 // per lane).
 template <int BLOCK, int K>
-__device__ __forceinline__ void bu_layout(const BfsParams &p, const StepView &sv, Local &loc)
+__device__ __forceinline__ void bu_layout(const BfsParams &p, const StepView &sv, const Team &team,
+                                          Local &loc)
 {
     if constexpr (K == 32) {
-        bu_step_lanes<BLOCK>(p, sv, loc);
+        bu_step_lanes<BLOCK>(p, sv, team, loc);
     } else {
-        bu_step<BLOCK, K>(p, sv, loc);
+        bu_step<BLOCK, K>(p, sv, team, loc);
     }
+}
+
+// ---------------------------------------------------------------------------
+// Narrow levels: CTA 0 alone
+// ---------------------------------------------------------------------------
+// A level of a few thousand arcs does not need the grid, and pays for it: the
+// grid barrier with its counters, and the round trips of a queue in global
+// memory.  CTA 0 therefore runs such levels by itself while the other CTAs wait
+// at one grid barrier.  Its queue lies in shared memory with each vertex's list
+// start, so a level is a chain of three round trips (arc; visited word; claim
+// with offsets) and a few block barriers.
+//
+// Levels of a 1021 x 1031 grid by frontier size, 512 threads, whole grid against
+// one CTA: up to 64 vertices 7.4 and 3.2 us, up to 256 8.6 and 4.3 us, up to 1024
+// 9.2 and 7.9 us, above 9.4 and 13.2 us (one SM's requests then bound it).  So the
+// line lies at kSoloArcs arcs (about 640 such vertices); kSoloCap keeps the
+// queues within the memory of the grid's own scratch, since a CTA that holds more
+// shared memory leaves less L1 for the bottom-up steps.  Bottom-up levels run here
+// in graphs of at most kSoloBu vertices while the lists of the unvisited ones hold
+// at most kSoloBuArcs arcs (1024 vertices: 28 -> 14 us for a whole search).
+// Levels before CTA 0 meets the others once, so that none polls for long.
+constexpr int kSoloLevels = 128;
+
+extern __shared__ __align__(16) unsigned char bfs_shared[];  // a SharedState
+
+template <int BLOCK>
+__device__ __forceinline__ bool solo_applies(const LevelState &st, const BfsParams &p)
+{
+    if (st.dir == kDirTD) {
+        return st.f_count <= kSoloCap<BLOCK> && st.f_degsum <= kSoloArcs<BLOCK>;
+    }
+    return st.dir == kDirBU && p.n <= kSoloBu<BLOCK> &&
+           2 * p.m - st.visited_degsum <= kSoloBuArcs<BLOCK>;
+}
+
+__device__ __forceinline__ uint32_t solo_hi(int64_t beg, int64_t deg)
+{
+    return ((uint32_t)((uint64_t)beg >> 32) << 16) | (uint32_t)min(deg, (int64_t)0xFFFF);
+}
+
+// Warp-collective: appends up to K vertices per lane to shared queue q; past its
+// end they go to the global queues (qout).
+template <int BLOCK, int K>
+__device__ __forceinline__ void solo_append(const BfsParams &p, SharedState<BLOCK> &sh,
+                                            SoloQueues<BLOCK> &sq, int q, int qout,
+                                            const bool (&has)[K], const uint32_t (&v)[K],
+                                            const int64_t (&beg)[K], const int64_t (&deg)[K],
+                                            Local &loc)
+{
+    unsigned m[K], total = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        m[k] = __ballot_sync(kFull, has[k]);
+        total += __popc(m[k]);
+    }
+    if (!total) { return; }
+    unsigned base = 0;
+    if (lane_id() == 0) { base = atomicAdd(&sh.queued, total); }
+    base = __shfl_sync(kFull, base, 0);
+    bool over[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const unsigned pos = base + __popc(m[k] & lanemask_lt());
+        base += __popc(m[k]);
+        over[k] = has[k] && pos >= (unsigned)kSoloCap<BLOCK>;
+        if (has[k]) {
+            loc.found += 1;
+            loc.degsum += (unsigned long long)deg[k];
+            if (!over[k]) {
+                sq.v[q][pos] = v[k];
+                sq.lo[q][pos] = (uint32_t)beg[k];
+                sq.hi[q][pos] = solo_hi(beg[k], deg[k]);
+            }
+        }
+    }
+    if (base > (unsigned)kSoloCap<BLOCK>) {
+        Local none{0, 0};
+        warp_append_k<K>(p, &sh.acc, qout, over, v, deg, none);
+    }
+}
+
+// The frontier of the state, from the global queues into shared queue q.
+template <int BLOCK>
+__device__ void solo_load(const BfsParams &p, SharedState<BLOCK> &sh, SoloQueues<BLOCK> &sq, int q)
+{
+    const LevelState &st = sh.st;
+    const int small = (int)st.f_small, count = (int)st.f_count;
+    for (int i = threadIdx.x; i < count; i += BLOCK) {
+        const uint32_t v = i < small ? __ldcg(&p.qs[st.q_cur][i]) : __ldcg(&p.ql[st.q_cur][i - small]);
+        const int64_t b = __ldg(&p.off[v]);
+        sq.v[q][i] = v;
+        sq.lo[q][i] = (uint32_t)b;
+        sq.hi[q][i] = solo_hi(b, __ldg(&p.off[v + 1]) - b);
+    }
+}
+
+// Shared queue q into the global queues of the state's frontier, beside what
+// has gone there already.
+template <int BLOCK>
+__device__ void solo_flush(const BfsParams &p, SharedState<BLOCK> &sh, SoloQueues<BLOCK> &sq, int q)
+{
+    const int count = (int)min(sh.queued, (unsigned)kSoloCap<BLOCK>);
+    Local none{0, 0};
+    for (int i0 = 0; i0 < count; i0 += BLOCK) {
+        const int i = i0 + threadIdx.x;
+        const bool has[1] = {i < count};
+        const uint32_t v[1] = {has[0] ? sq.v[q][i] : 0u};
+        int64_t deg[1] = {has[0] ? (int64_t)(sq.hi[q][i] & 0xFFFFu) : 0};
+        if (deg[0] == 0xFFFF) { deg[0] = degree_of(p, v[0]); }
+        warp_append_k<1>(p, &sh.acc, sh.st.q_cur, has, v, deg, none);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        LevelState &st = sh.st;
+        st.f_small = (long long)sh.acc.small_cnt;
+        st.f_large = (long long)(sh.acc.large_packed >> kLargeShift);
+        st.f_chunks = (long long)(sh.acc.large_packed & kChunkMask);
+    }
+}
+
+// Degrees in the low halves of hi[q] become positions of the lists' first arcs.
+template <int BLOCK>
+__device__ void solo_scan(SharedState<BLOCK> &sh, SoloQueues<BLOCK> &sq, int q, int count)
+{
+    constexpr int E = (kSoloCap<BLOCK> + BLOCK - 1) / BLOCK;  // consecutive entries per thread
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    uint32_t h[E];
+    unsigned sum = 0;
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const int i = (int)threadIdx.x * E + k;
+        h[k] = i < count ? sq.hi[q][i] : 0u;
+        sum += h[k] & 0xFFFFu;
+    }
+    const unsigned incl = warp_incl_scan(sum);
+    if (lane == 31) { sh.warp_sum[warp] = incl; }
+    __syncthreads();
+    const unsigned w = lane < BLOCK / 32 ? sh.warp_sum[lane] : 0u;
+    const unsigned wi = warp_incl_scan(w);
+    unsigned at = incl - sum + (warp ? __shfl_sync(kFull, wi, warp - 1) : 0u);
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const int i = (int)threadIdx.x * E + k;
+        if (i < count) { sq.hi[q][i] = (h[k] & 0xFFFF0000u) | at; }
+        at += h[k] & 0xFFFFu;
+    }
+    __syncthreads();
+}
+
+// A top-down level from shared queue q into q ^ 1.  The arcs of all lists, laid
+// end to end, are dealt to the threads, ILP at a time with each stage's reads
+// issued together; an unvisited neighbour is claimed by the atomicOr on its
+// visited word (its old value names the one winner), and its offsets are read
+// with the claim rather than after it.
+template <int BLOCK, int ILP>
+__device__ __forceinline__ void solo_td(const BfsParams &p, SharedState<BLOCK> &sh, SoloQueues<BLOCK> &sq, int q,
+                        Local &loc)
+{
+    const LevelState &st = sh.st;
+    const int count = (int)st.f_count, arcs = (int)st.f_degsum, new_level = st.level + 1;
+    const int qout = st.q_cur ^ 1;
+    uint32_t *vis = p.vis[st.vis_cur];
+    int top = 1;  // first step of the searches: the largest power of two below count
+    while (top * 2 < count) { top *= 2; }
+    // whole warps: the appends are warp-collective
+    for (int e0 = (int)threadIdx.x & ~31; e0 < arcs; e0 += BLOCK * ILP) {
+        bool won[ILP];
+        int e[ILP], at[ILP];
+        uint32_t v[ILP], src[ILP];
+        int64_t beg[ILP], deg[ILP];
+#pragma unroll
+        for (int i = 0; i < ILP; ++i) {
+            e[i] = e0 + i * BLOCK + lane_id();
+            won[i] = e[i] < arcs;
+            at[i] = 0;  // last list that starts at or before arc e
+        }
+        for (int d = top; d > 0; d >>= 1) {
+#pragma unroll
+            for (int i = 0; i < ILP; ++i) {
+                const int t = at[i] + d;
+                if (t < count && (int)(sq.hi[q][t] & 0xFFFFu) <= e[i]) { at[i] = t; }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < ILP; ++i) {
+            const uint32_t h = sq.hi[q][at[i]];
+            const int64_t b = ((int64_t)(h >> 16) << 32) | sq.lo[q][at[i]];
+            src[i] = sq.v[q][at[i]];
+            v[i] = won[i] ? __ldg(&p.adj[b + (e[i] - (int)(h & 0xFFFFu))]) : 0u;
+        }
+        uint32_t old[ILP];
+#pragma unroll
+        for (int i = 0; i < ILP; ++i) { old[i] = won[i] ? __ldcg(&vis[v[i] >> 5]) : 0xFFFFFFFFu; }
+#pragma unroll
+        for (int i = 0; i < ILP; ++i) {
+            won[i] = !((old[i] >> (v[i] & 31)) & 1u);
+            beg[i] = deg[i] = 0;
+            if (won[i]) {
+                old[i] = atomicOr(&vis[v[i] >> 5], 1u << (v[i] & 31));
+                beg[i] = __ldg(&p.off[v[i]]);
+                deg[i] = __ldg(&p.off[v[i] + 1]) - beg[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < ILP; ++i) {
+            won[i] = won[i] && !((old[i] >> (v[i] & 31)) & 1u);
+            if (won[i]) {
+                p.depth[v[i]] = new_level;
+                p.parent[v[i]] = (int64_t)src[i];
+            }
+        }
+        solo_append<BLOCK, ILP>(p, sh, sq, q ^ 1, qout, won, v, beg, deg, loc);
+    }
+}
+
+// The source frontier (hybrid_bfs.cc:158-163 for one source; any number of
+// sources start as one frontier) into shared queue 0, and the first decision.
+template <int BLOCK>
+__device__ void solo_init(const BfsParams &p, SharedState<BLOCK> &sh, SoloQueues<BLOCK> &sq,
+                          Local &loc)
+{
+    for (int64_t i0 = (int64_t)(threadIdx.x & ~31u); i0 < p.source_count; i0 += BLOCK) {
+        const int64_t i = i0 + lane_id();
+        bool has[1] = {i < p.source_count};
+        uint32_t v[1] = {0u};
+        int64_t beg[1] = {0}, deg[1] = {0};
+        if (has[0]) {
+            const int64_t s = p.sources ? __ldg(&p.sources[i]) : p.source;
+            v[0] = p.perm ? __ldg(&p.perm[s]) : (uint32_t)s;
+            beg[0] = __ldg(&p.off[v[0]]);
+            deg[0] = __ldg(&p.off[v[0] + 1]) - beg[0];
+            has[0] = atomicCAS(&p.depth[v[0]], -1, 0) == -1;  // else a repeated source
+        }
+        if (has[0]) {
+            p.parent[v[0]] = (int64_t)v[0];
+            atomicOr(&p.vis[0][v[0] >> 5], 1u << (v[0] & 31));
+        }
+        solo_append<BLOCK, 1>(p, sh, sq, 0, 0, has, v, beg, deg, loc);
+    }
+    unsigned long long tf, td;
+    block_totals<BLOCK>(sh, loc, tf, td);
+    if (threadIdx.x == 0) {
+        LevelState &st = sh.st;
+        st.f_count = (long long)tf;
+        st.f_degsum = (long long)td;
+        st.visited_degsum = (long long)td;
+        st.reached = (long long)tf;
+        st.etc = 2 * p.m;             // edges_to_check = num_edges * 2
+        st.scout = (long long)td;     // scout_count = out_degree(source)
+        st.prev_dir = kDirTD;
+        st.t_last = globaltimer();
+        decide_rule(st, p, sh.rule_dir, sh.consult);
+    }
+    __syncthreads();
+    decide_policy(p, sh);
+}
+
+// CTA 0: the source setup (init), then levels as long as they are narrow.  Not
+// inlined: beside it the grid's steps would spill registers (12 % slower
+// bottom-up and top-down levels at scales 19 and 22).
+template <int BLOCK>
+__device__ __noinline__ void solo_run(bool init)
+{
+    SharedState<BLOCK> &sh = *reinterpret_cast<SharedState<BLOCK> *>(bfs_shared);
+    const BfsParams &p = sh.par;
+    SoloQueues<BLOCK> &sq = sh.queues;
+    Local loc{0, 0};
+    int q = 0;
+    bool shared_queue = init;  // the frontier is in queue q (else in the global queues)
+    if (threadIdx.x == 0) {
+        sh.queued = 0;
+        sh.acc.small_cnt = sh.acc.large_packed = 0;
+    }
+    __syncthreads();
+    if (init) { solo_init<BLOCK>(p, sh, sq, loc); }
+    for (int l = 0; l < kSoloLevels && solo_applies<BLOCK>(sh.st, p); ++l) {
+        if (sh.st.dir == kDirTD) {
+            if (!shared_queue) {
+                solo_load<BLOCK>(p, sh, sq, q);
+                __syncthreads();
+            }
+            solo_scan<BLOCK>(sh, sq, q, (int)sh.st.f_count);
+            if (threadIdx.x == 0) { sh.queued = 0; }
+            __syncthreads();
+            if (sh.st.f_degsum <= BLOCK) {  // one arc a thread: four slots would issue for nothing
+                solo_td<BLOCK, 1>(p, sh, sq, q, loc);
+            } else {
+                solo_td<BLOCK, kILP>(p, sh, sq, q, loc);
+            }
+            q ^= 1;
+            shared_queue = true;
+        } else {
+            if (threadIdx.x == 0) { sh.queued = 0; }
+            const StepView sv = view_of(sh.st);
+            const Team team{(long long)(threadIdx.x >> 5), BLOCK / 32, &sh.acc};
+            bu_step<BLOCK, 1>(p, sv, team, loc);
+            shared_queue = false;
+        }
+        unsigned long long tf, td;
+        block_totals<BLOCK>(sh, loc, tf, td);
+        if (threadIdx.x == 0) {
+            LevelState &st = sh.st;
+            const long long t_end = globaltimer();
+            Acc a;
+            a.found = tf;
+            a.degsum = td;
+            a.small_cnt = sh.acc.small_cnt;
+            a.large_packed = sh.acc.large_packed;
+            record_step(p, st, (long long)tf, t_end);
+            advance(st, p, a, t_end);
+            decide_rule(st, p, sh.rule_dir, sh.consult);
+            // what lies in the global queues counts for this frontier only
+            if (!shared_queue || solo_applies<BLOCK>(st, p)) {
+                sh.acc.small_cnt = sh.acc.large_packed = 0;
+            }
+        }
+        __syncthreads();
+        decide_policy(p, sh);
+    }
+    if (shared_queue && sh.st.dir != kDirDone) { solo_flush<BLOCK>(p, sh, sq, q); }
 }
 
 // KD: bottom-up layout while most live vertices are unvisited; KS: after.
 template <int BLOCK, int MINB, int KD, int KS>
-__global__ void __launch_bounds__(BLOCK, MINB) bfs_persistent_kernel(BfsParams p)
+__global__ void __launch_bounds__(BLOCK, MINB) bfs_persistent_kernel(
+    const __grid_constant__ BfsParams p)
 {
-    __shared__ SharedState<BLOCK> sh;
+    SharedState<BLOCK> &sh = *reinterpret_cast<SharedState<BLOCK> *>(bfs_shared);
     Ctrl *c = p.ctrl;
-    if (threadIdx.x == 0) {
-        sh.st = c->st;  // written by the init kernel before this launch
-        atomicMin(&c->t_start, (unsigned long long)globaltimer());
-    }
     if (p.policy) {
         const float *src = reinterpret_cast<const float *>(p.policy);
         float *dst = reinterpret_cast<float *>(&sh.pol);
@@ -836,79 +1239,70 @@ __global__ void __launch_bounds__(BLOCK, MINB) bfs_persistent_kernel(BfsParams p
             dst[i] = src[i];
         }
     }
+    if (threadIdx.x == 0) {
+        memset(&sh.st, 0, sizeof(LevelState));
+        sh.par = p;
+        sh.st.barrier = c->barrier;
+        // an earlier launch of the call timed out: its barrier count is void
+        sh.consult = __ldcg(&c->error);
+    }
     __syncthreads();
+    if (sh.consult) { return; }
+    const Team grid{(long long)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5),
+                    (long long)gridDim.x * (BLOCK / 32), nullptr};
+    bool init = true;
     Local loc{0, 0};
-    while (sh.st.dir != kDirDone) {
+    do {
+        if (init || solo_applies<BLOCK>(sh.st, p)) {
+            // CTA 0 alone; the others take the state it publishes
+            if (blockIdx.x == 0) { solo_run<BLOCK>(init); }
+            init = false;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const long long b = sh.st.barrier;
+                if (blockIdx.x == 0) {
+                    c->pub[b & 1] = sh.st;
+                    clear_next_acc(c, b);
+                }
+                if (arrive_wait(p, b, blockIdx.x != 0)) {
+                    if (blockIdx.x != 0) {
+                        const long long *from = reinterpret_cast<const long long *>(&c->pub[b & 1]);
+                        long long *to = reinterpret_cast<long long *>(&sh.st);
+#pragma unroll
+                        for (int i = 0; i < (int)(sizeof(LevelState) / 8); ++i) {
+                            to[i] = __ldcg(&from[i]);
+                        }
+                    }
+                } else {
+                    sh.st.dir = kDirDone;
+                }
+                sh.st.barrier = b + 1;
+            }
+            __syncthreads();
+            continue;
+        }
         const StepView sv = view_of(sh.st);
+        Team team = grid;
+        team.acc = &c->acc[sv.barrier % 3];
         if (sv.dir == kDirTD) {
-            td_step<BLOCK>(p, sv, sh, loc);
+            td_step<BLOCK>(p, sv, team, sh, loc);
         } else {
             if (sv.bu_sparse) {
-                bu_layout<BLOCK, KS>(p, sv, loc);
+                bu_layout<BLOCK, KS>(p, sv, team, loc);
             } else {
-                bu_layout<BLOCK, KD>(p, sv, loc);
+                bu_layout<BLOCK, KD>(p, sv, team, loc);
             }
         }
         end_step<BLOCK>(p, sv, sh, loc);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) { c->st = sh.st; }
-}
-
-struct InitShared {
-    int rule_dir;
-    LevelState st;
-};
-
-// clear() + the source frontier (hybrid_bfs.cc:152-160 for one source; any
-// number of sources start as one frontier), and the first decision.  One
-// CTA of 32 threads.
-__global__ void init_sources_kernel(BfsParams p, const int64_t *sources, int64_t count,
-                                    int64_t source_index)
-{
-    __shared__ InitShared sh;
-    Ctrl *c = p.ctrl;
-    if (threadIdx.x == 0) {
-        memset(c, 0, sizeof(Ctrl));
-        c->t_start = ~0ull;
-        LevelState &st = sh.st;
-        memset(&st, 0, sizeof(LevelState));
-        long long degsum = 0, nf = 0, nsmall = 0;
-        unsigned long long lp = 0;
-        const int64_t first = source_index >= 0 ? source_index : 0;
-        const int64_t last = source_index >= 0 ? source_index + 1 : count;
-        for (int64_t i = first; i < last; ++i) {
-            const uint32_t s = p.perm ? p.perm[sources[i]] : (uint32_t)sources[i];
-            if (p.depth[s] == 0) { continue; }  // repeated source
-            p.depth[s] = 0;
-            p.parent[s] = (int64_t)s;
-            p.vis[0][s >> 5] |= 1u << (s & 31);
-            const int64_t deg = p.off[s + 1] - p.off[s];
-            degsum += deg;
-            nf += 1;
-            if (deg >= (int64_t)p.large_deg) {
-                const unsigned long long pos = lp >> kLargeShift;
-                p.ql[0][pos] = s;
-                p.qlb[0][pos] = lp & kChunkMask;
-                lp += (1ull << kLargeShift) | (unsigned long long)((deg + p.chunk - 1) / p.chunk);
-            } else {
-                p.qs[0][nsmall++] = s;
-            }
+    } while (sh.st.dir != kDirDone);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        c->st = sh.st;
+        c->barrier = sh.st.barrier;
+        if (p.result) {
+            p.result[0] = sh.st.visited_degsum / 2;
+            p.result[1] = sh.st.reached;
         }
-        st.f_count = nf;
-        st.f_degsum = degsum;
-        st.f_small = nsmall;
-        st.f_large = (long long)(lp >> kLargeShift);
-        st.f_chunks = (long long)(lp & kChunkMask);
-        st.visited_degsum = degsum;
-        st.reached = nf;
-        st.etc = 2 * p.m;       // edges_to_check = num_edges * 2
-        st.scout = degsum;      // scout_count = out_degree(source)
-        st.prev_dir = kDirTD;
     }
-    __syncthreads();
-    decide_next(sh.st, p, p.policy, sh);
-    __syncthreads();
-    if (threadIdx.x == 0) { c->st = sh.st; }
 }
 
 // Deterministic tree: parent(v) = min{u in N(v) : depth[u] == depth[v]-1}.
@@ -990,10 +1384,15 @@ __global__ void hub_outputs_kernel(const uint32_t *perm, const uint32_t *iperm, 
     }
 }
 
-__global__ void save_result_kernel(const Ctrl *c, int64_t *out, int64_t i)
+// clear(): no vertex visited but the isolated ones.
+__global__ void clear_kernel(int64_t n, const uint32_t *isolated, int32_t *depth, uint32_t *vis)
 {
-    out[2 * i] = c->st.visited_degsum / 2;
-    out[2 * i + 1] = c->st.reached;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+    int4 *d4 = reinterpret_cast<int4 *>(depth);  // cudaMalloc aligns to 256
+    for (int64_t i = t; i < n / 4; i += nt) { d4[i] = make_int4(-1, -1, -1, -1); }
+    if (t < (n & 3)) { depth[(n & ~(int64_t)3) + t] = -1; }
+    for (int64_t w = t; w < (n + 31) / 32; w += nt) { vis[w] = isolated[w]; }
 }
 
 int grid_for(int64_t items, int threads = 256)
@@ -1009,19 +1408,35 @@ using KernelFn = void (*)(BfsParams);
 struct KernelChoice {
     KernelFn fn;
     int block;
+    size_t smem;  // dynamic shared memory
 };
 
 KernelChoice pick_kernel(int block, int kd = 4, int ks = 4)
 {
 #define BD_KC(B, M, D, S) \
-    if (block == B && kd == D && ks == S) { return {bfs_persistent_kernel<B, M, D, S>, B}; }
+    if (block == B && kd == D && ks == S) { return {bfs_persistent_kernel<B, M, D, S>, B, sizeof(SharedState<B>)}; }
 #define BD_KC_B(B, M)                                                                  \
     BD_KC(B, M, 1, 1) BD_KC(B, M, 2, 2) BD_KC(B, M, 4, 4) BD_KC(B, M, 32, 32)          \
     BD_KC(B, M, 2, 32) BD_KC(B, M, 4, 32)
     BD_KC_B(256, 4) BD_KC_B(512, 2) BD_KC_B(1024, 1)
 #undef BD_KC_B
 #undef BD_KC
-    return {nullptr, 0};
+    return {nullptr, 0, 0};
+}
+
+// Allows the kernel its shared memory and returns the CTAs of the device that
+// can be resident at once (0 after an error).
+int co_resident_ctas(const KernelChoice &kc, int device)
+{
+    int per_sm = 0, sms = 0;
+    if (cudaFuncSetAttribute((const void *)kc.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kc.smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)kc.fn, kc.block,
+                                                      kc.smem) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        return 0;
+    }
+    return per_sm * sms;
 }
 
 }  // namespace
@@ -1047,9 +1462,9 @@ struct bd_bfs {
     int64_t *d_sources = nullptr;
     int64_t sources_cap = 0;
     PolicyBlob *policy = nullptr;  // device copy, or null
-    KernelFn kernel = nullptr;
-    int block = 512;
+    KernelChoice kernel{nullptr, 0, 0};
     int grid = 0;
+    bool ctrl_valid = false;  // no launch has failed since the control block was zeroed
     int64_t cap_large = 0;
     // BD_ORDER_HUB graphs: depths and parents in the caller's numbering,
     // filled from the traversal arrays when first read after a run
@@ -1116,10 +1531,9 @@ BfsParams make_params(bd_bfs *b)
 bd_status enqueue_clear(bd_bfs *b)
 {
     const int64_t n = b->g->n;
-    BD_CUDA(cudaMemsetAsync(b->depth, 0xFF, sizeof(int32_t) * n, b->stream));
-    BD_CUDA(cudaMemcpyAsync(b->vis[0], traversal_isolated(b->g),
-                            sizeof(uint32_t) * bitmap_words(n), cudaMemcpyDeviceToDevice,
-                            b->stream));
+    clear_kernel<<<grid_for(n, 512), 256, 0, b->stream>>>(n, traversal_isolated(b->g), b->depth,
+                                                          b->vis[0]);
+    BD_CUDA(cudaGetLastError());
     return BD_OK;
 }
 
@@ -1152,23 +1566,29 @@ __global__ void copy_outputs_kernel(const int64_t *off, int64_t n, const int32_t
     }
 }
 
-// Enqueues init + the persistent kernel (+ min-parent pass) for either a
-// set of sources (index < 0) or source d_sources[index].  With out_depth /
-// out_parent (device, n entries each) the results are also written there
+// Enqueues the persistent kernel (+ min-parent pass) for `count` sources in
+// d_sources, or for the one source given (count 1).  m_c and n_c go to result
+// (device) if given.  With out_depth / out_parent (device, n entries each) the results are also written there
 // in the caller's ids and the reference's encoding, inside the timed region.
-bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t index, cudaEvent_t start,
-                      cudaEvent_t stop, int32_t *out_depth = nullptr,
+bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t start,
+                      cudaEvent_t stop, int64_t *result = nullptr, int32_t *out_depth = nullptr,
                       int64_t *out_parent = nullptr)
 {
     BfsParams p = make_params(b);
+    p.sources = count > 1 ? b->d_sources : nullptr;
+    p.source = source;
+    p.source_count = count;
+    p.result = result;
+    if (!b->ctrl_valid) {
+        BD_CUDA(cudaMemsetAsync(b->ctrl, 0, sizeof(Ctrl), b->stream));
+        b->ctrl_valid = true;
+    }
     // The timed region starts with the source setup, as run_beamer's does
     // (hybrid_bfs.cc:158-160); clear() stays outside it.
     if (start) { BD_CUDA(cudaEventRecord(start, b->stream)); }
-    init_sources_kernel<<<1, 32, 0, b->stream>>>(p, b->d_sources, count, index);
-    BD_CUDA(cudaGetLastError());
     void *args[] = {&p};
-    BD_CUDA(cudaLaunchCooperativeKernel((const void *)b->kernel, dim3(b->grid), dim3(b->block),
-                                        args, 0, b->stream));
+    BD_CUDA(cudaLaunchCooperativeKernel((const void *)b->kernel.fn, dim3(b->grid),
+                                        dim3(b->kernel.block), args, b->kernel.smem, b->stream));
     if (out_depth) {
         const int64_t n = b->g->n;
         if (b->g->d_perm) {
@@ -1215,7 +1635,10 @@ bd_status collect(bd_bfs *b, bd_run_stats *stats, double ms)
     b->cleared = false;
     // a min-parent run on a hub graph wrote the caller-order outputs itself
     b->parents_final = b->out_depth != nullptr && b->opts.min_parent;
-    if (b->last.error) { return (bd_status)b->last.error; }
+    if (b->last.error) {
+        b->ctrl_valid = false;
+        return (bd_status)b->last.error;
+    }
     if (stats) {
         stats->ms = ms;
         stats->num_steps = b->last.st.step;
@@ -1234,11 +1657,13 @@ bd_status run_sources(bd_bfs *b, const int64_t *sources, int64_t count, bd_run_s
         if (sources[i] < 0 || sources[i] >= b->g->n) { return BD_ERR_RANGE; }
     }
     BD_CUDA(cudaSetDevice(b->device));
-    BD_TRY(ensure_sources(b, count));
     if (!b->cleared) { BD_TRY(enqueue_clear(b)); }
-    BD_CUDA(cudaMemcpyAsync(b->d_sources, sources, sizeof(int64_t) * count,
-                            cudaMemcpyHostToDevice, b->stream));
-    BD_TRY(enqueue_bfs(b, count, -1, b->ev0, b->ev1));
+    if (count > 1) {
+        BD_TRY(ensure_sources(b, count));
+        BD_CUDA(cudaMemcpyAsync(b->d_sources, sources, sizeof(int64_t) * count,
+                                cudaMemcpyHostToDevice, b->stream));
+    }
+    BD_TRY(enqueue_bfs(b, count, sources[0], b->ev0, b->ev1));
     BD_CUDA(cudaEventSynchronize(b->ev1));
     float ms = 0.f;
     BD_CUDA(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
@@ -1360,18 +1785,10 @@ bd_status bd_bfs_create(bd_graph *g, const bd_bfs_opts *opts, bd_bfs **out)
              cudaMalloc(&b->qlb[i], sizeof(unsigned long long) * b->cap_large) == cudaSuccess;
     }
     if (!ok) { return fail(BD_ERR_OOM); }
-    KernelChoice kc = pick_kernel(o.block_size, o.bu_words, o.bu_sparse_words);
-    if (!kc.fn) { return fail(BD_ERR_INVALID); }
-    b->kernel = kc.fn;
-    b->block = kc.block;
-    int per_sm = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)b->kernel, b->block, 0) !=
-            cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess ||
-        per_sm < 1) {
-        return fail(BD_ERR_CUDA);
-    }
-    b->grid = per_sm * sms;
+    b->kernel = pick_kernel(o.block_size, o.bu_words, o.bu_sparse_words);
+    if (!b->kernel.fn) { return fail(BD_ERR_INVALID); }
+    b->grid = co_resident_ctas(b->kernel, b->device);
+    if (b->grid < 1) { return fail(BD_ERR_CUDA); }
     *out = b;
     return BD_OK;
 }
@@ -1443,7 +1860,6 @@ bd_status run_many(bd_bfs *b, const int64_t *sources, int64_t k, int32_t *d_dept
         if (sources[i] < 0 || sources[i] >= b->g->n) { return BD_ERR_RANGE; }
     }
     BD_CUDA(cudaSetDevice(b->device));
-    BD_TRY(ensure_sources(b, k));
     int64_t *d_edges = nullptr;
     std::vector<cudaEvent_t> ev(2 * k, nullptr);
     bd_status st = BD_OK;
@@ -1464,21 +1880,13 @@ bd_status run_many(bd_bfs *b, const int64_t *sources, int64_t k, int32_t *d_dept
     }
     std::vector<int64_t> host_edges(2 * k);
     cudaEventRecord(wall0, b->stream);
-    if (cudaMemcpyAsync(b->d_sources, sources, sizeof(int64_t) * k, cudaMemcpyHostToDevice,
-                        b->stream) != cudaSuccess) {
-        cleanup();
-        return BD_ERR_CUDA;
-    }
     const int64_t n = b->g->n;
     for (int64_t i = 0; i < k && st == BD_OK; ++i) {
         st = enqueue_clear(b);
         if (st == BD_OK) {
-            st = enqueue_bfs(b, k, i, ev[2 * i], ev[2 * i + 1], d_depth ? d_depth + i * n : nullptr,
+            st = enqueue_bfs(b, 1, sources[i], ev[2 * i], ev[2 * i + 1], d_edges + 2 * i,
+                             d_depth ? d_depth + i * n : nullptr,
                              d_depth ? d_parent + i * n : nullptr);
-        }
-        if (st == BD_OK) {
-            save_result_kernel<<<1, 1, 0, b->stream>>>(b->ctrl, d_edges, i);
-            if (cudaGetLastError() != cudaSuccess) { st = BD_ERR_CUDA; }
         }
     }
     if (st == BD_OK &&
@@ -1619,8 +2027,7 @@ constexpr int64_t kNaWords = kNaMaxVertices / 32;
 constexpr int64_t kNaLarge = 1 << 17;  // slots for large-degree frontier vertices
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kNaOffCtrl = 0;
-constexpr size_t kNaOffSource = align256(kNaOffCtrl + sizeof(Ctrl));
-constexpr size_t kNaOffLive = kNaOffSource + sizeof(int64_t);  // vertices of nonzero degree
+constexpr size_t kNaOffLive = align256(kNaOffCtrl + sizeof(Ctrl));  // vertices of nonzero degree
 constexpr size_t kNaOffVis = align256(kNaOffLive + sizeof(unsigned long long));
 constexpr size_t kNaOffQs = align256(kNaOffVis + 2 * sizeof(uint32_t) * kNaWords);
 constexpr size_t kNaOffQl = align256(kNaOffQs + 2 * sizeof(uint32_t) * kNaMaxVertices);
@@ -1645,13 +2052,9 @@ bd_status noalloc_setup(int dev, unsigned char **base, int *grid)
         void *ptr = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
         if (e != cudaSuccess) { return cuda_fail(e, "cudaGetSymbolAddress", __FILE__, __LINE__); }
-        int per_sm = 0, sms = 0;
-        KernelChoice kc = pick_kernel(512);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)kc.fn, kc.block, 0);
-        if (e == cudaSuccess) { e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-        if (e != cudaSuccess) { return cuda_fail(e, "occupancy", __FILE__, __LINE__); }
-        if (per_sm < 1) { return BD_ERR_CUDA; }
-        g_na_grid[dev] = per_sm * sms;
+        const int ctas = co_resident_ctas(pick_kernel(512), dev);
+        if (ctas < 1) { return cuda_fail(cudaGetLastError(), "occupancy", __FILE__, __LINE__); }
+        g_na_grid[dev] = ctas;
         g_na_base[dev] = static_cast<unsigned char *>(ptr);
     }
     *base = g_na_base[dev];
@@ -1659,11 +2062,10 @@ bd_status noalloc_setup(int dev, unsigned char **base, int *grid)
     return BD_OK;
 }
 
-// depth = -1; vis[0] = degree-zero and padding bits; the source id; the
-// count of vertices of nonzero degree added into *live (zeroed before).
+// depth = -1; vis[0] = degree-zero and padding bits; the count of vertices of
+// nonzero degree added into *live (zeroed before).
 __global__ void noalloc_prepare_kernel(const int64_t *off, int64_t n, int32_t *depth,
-                                       uint32_t *vis0, int64_t source, int64_t *source_slot,
-                                       unsigned long long *live)
+                                       uint32_t *vis0, unsigned long long *live)
 {
     const int64_t words = (n + 31) / 32;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1681,7 +2083,6 @@ __global__ void noalloc_prepare_kernel(const int64_t *off, int64_t n, int32_t *d
     }
     nz = dev::warp_sum(nz);
     if (dev::lane_id() == 0 && nz) { atomicAdd(live, nz); }
-    if (t == 0) { *source_slot = source; }
 }
 
 }  // namespace
@@ -1718,7 +2119,6 @@ extern "C" bd_status bd_bfs_run_noalloc(const int64_t *d_offsets, const uint32_t
     p.parent = d_parent;
     p.words = bitmap_words(num_vertices);
     Ctrl *ctrl = reinterpret_cast<Ctrl *>(base + kNaOffCtrl);
-    int64_t *source_slot = reinterpret_cast<int64_t *>(base + kNaOffSource);
     unsigned long long *live = reinterpret_cast<unsigned long long *>(base + kNaOffLive);
     for (int i = 0; i < 2; ++i) {
         p.vis[i] = reinterpret_cast<uint32_t *>(base + kNaOffVis) + i * kNaWords;
@@ -1742,24 +2142,26 @@ extern "C" bd_status bd_bfs_run_noalloc(const int64_t *d_offsets, const uint32_t
     p.spin_limit = kDefaultSpin;
     p.expected_ctas = (unsigned)grid;
     p.policy = nullptr;
+    p.source = source;
+    p.source_count = 1;
 
-    // The control block, source slot, live count and vis[0] are rewritten
+    // The control block, live count and vis[0] are rewritten
     // here; the queues and vis[1] are written before they are read within a
     // run.  The live count (vertices of nonzero degree) decides the
     // bottom-up layout switch, so it is read back before the launch.
-    BD_CUDA(cudaMemsetAsync(live, 0, sizeof(unsigned long long), s));
+    BD_CUDA(cudaMemsetAsync(base + kNaOffCtrl, 0,
+                            kNaOffLive + sizeof(unsigned long long) - kNaOffCtrl, s));
     noalloc_prepare_kernel<<<grid_for(std::max<int64_t>(num_vertices, 1)), 256, 0, s>>>(
-        d_offsets, num_vertices, d_depth, p.vis[0], source, source_slot, live);
+        d_offsets, num_vertices, d_depth, p.vis[0], live);
     BD_CUDA(cudaGetLastError());
     unsigned long long n_live = 0;
     BD_CUDA(cudaMemcpyAsync(&n_live, live, sizeof(n_live), cudaMemcpyDeviceToHost, s));
     BD_CUDA(cudaStreamSynchronize(s));
     p.n_live = (int64_t)n_live;
-    init_sources_kernel<<<1, 32, 0, s>>>(p, source_slot, 1, 0);
-    BD_CUDA(cudaGetLastError());
     KernelChoice kc = pick_kernel(512);
     void *args[] = {&p};
-    BD_CUDA(cudaLaunchCooperativeKernel((const void *)kc.fn, dim3(grid), dim3(kc.block), args, 0, s));
+    BD_CUDA(cudaLaunchCooperativeKernel((const void *)kc.fn, dim3(grid), dim3(kc.block), args,
+                                        kc.smem, s));
     finalize_parents_kernel<<<grid_for(num_vertices), 256, 0, s>>>(d_offsets, num_vertices, d_depth,
                                                                    d_parent);
     BD_CUDA(cudaGetLastError());

@@ -5,7 +5,9 @@
 // or a bottom-up step (visited-bitmap scan with early exit), followed by a
 // grid barrier (one release-add per CTA, acquire polling) after which every
 // CTA reads the step's counters and makes the same direction decision for
-// the next level.  No host round trip happens inside a BFS.
+// the next level.  The source setup and levels too narrow to occupy the grid
+// are run by CTA 0 alone, with block barriers only, while the others wait at
+// one grid barrier (solo_run).  No host round trip happens inside a BFS.
 //
 // Reference counterparts:
 //   run_beamer                hybrid_bfs.cc:152-191   (decide_next / beamer_*)
@@ -28,9 +30,11 @@ constexpr int kDirDone = 2;
 constexpr int kLargeShift = 38;  // large-queue counter: count << 38 | chunks
 constexpr unsigned long long kChunkMask = (1ull << kLargeShift) - 1;
 
-// Counters the CTAs accumulate during one step, in a ring of three slots:
-// step s uses slot s % 3, CTA 0 clears slot (s + 1) % 3 during step s (every
-// CTA finished reading it before arriving at the barrier of step s - 1).
+// Counters the CTAs accumulate during one step, in a ring of three slots: the
+// step that ends at grid barrier b uses slot b % 3, CTA 0 clears slot
+// (b + 1) % 3 before it arrives there (every CTA finished reading it before
+// arriving at barrier b - 1).  Barriers are numbered through from launch to
+// launch, so a launch finds its first slot clear.
 struct Acc {
     unsigned long long found;
     unsigned long long degsum;
@@ -40,10 +44,10 @@ struct Acc {
     unsigned long long pad[3];
 };
 
-// The traversal state between steps.  The init kernel writes the first one
-// into Ctrl; every CTA then keeps an identical copy in shared memory and
-// advances it with the same function of the same counters after each
-// barrier; CTA 0 writes the final one back for the host.
+// The traversal state between steps.  CTA 0 publishes the first one (and the
+// one after each run of narrow levels); every CTA then keeps an identical copy
+// in shared memory and advances it with the same function of the same counters
+// after each barrier; CTA 0 writes the final one back for the host.
 struct LevelState {
     int dir;        // direction of the step about to run, or kDirDone
     int level;      // depth of the current frontier
@@ -64,15 +68,17 @@ struct LevelState {
     long long reached;
     long long td_steps, bu_steps;
     long long policy_overrides;  // learned decisions that differed from Beamer
+    long long barrier;           // number of the next grid barrier
 };
 
 // Device-resident control block of one BFS handle.
 struct Ctrl {
-    unsigned long long bar;      // barrier arrivals; step s is complete at (s+1) * CTAs
+    unsigned long long bar;      // arrivals; barrier b is complete at (b + 1) * CTAs
     int error;
     int pad0;
-    unsigned long long t_start;  // min over CTAs of their start time
-    LevelState st;
+    long long barrier;           // number of the next launch's first barrier
+    LevelState st;               // the final state, for the host
+    LevelState pub[2];           // published by CTA 0 at barrier b, in slot b % 2
     Acc acc[3];
 };
 
@@ -102,6 +108,10 @@ struct BfsParams {
     unsigned expected_ctas;
     const PolicyBlob *policy;  // null: no learned policy loaded
     const uint32_t *perm;      // caller id -> traversal id (BD_ORDER_HUB), or null
+    const int64_t *sources;    // device array of source_count caller ids, or null:
+    int64_t source;            // the one source
+    int64_t source_count;
+    int64_t *result;           // null, or where m_c and n_c of the run go
 };
 
 }  // namespace bd

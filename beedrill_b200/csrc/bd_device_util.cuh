@@ -15,6 +15,14 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
     return v;
 }
 
+// A poll without the acquire's effect on the SM's L1 (bd_bfs.cu, arrive_wait).
+__device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // Arrival at a grid barrier: orders every write the CTA made before it (the
 // CTA synchronised with __syncthreads first) ahead of the increment.
 __device__ __forceinline__ void red_release_add64(unsigned long long *p, unsigned long long v)

@@ -742,7 +742,7 @@ __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
     }
 }
 
-// Grid barrier: arrival (one release-add per CTA) and acquire polling until
+// Grid barrier: arrival (one release-add per CTA) and polling until
 // every CTA has arrived.  Bounded by p.spin_limit polls.  Thread 0 of each CTA;
 // b is the number of barriers passed before.
 __device__ __forceinline__ bool ms_arrive_wait(const MsParams &p, long long b)
