@@ -1305,48 +1305,152 @@ __global__ void __launch_bounds__(BLOCK, MINB) bfs_persistent_kernel(
     }
 }
 
-// Deterministic tree: parent(v) = min{u in N(v) : depth[u] == depth[v]-1}.
-// Warp per 32 vertices; short lists per lane, long lists by the whole warp.
-__global__ void min_parent_kernel(const int64_t *off, const uint32_t *adj, int64_t n,
-                                  const int32_t *depth, int64_t *parent)
+// ---------------------------------------------------------------------------
+// Deterministic tree: parent(v) = min{u in N(v) : depth[u] == depth[v]-1}
+// ---------------------------------------------------------------------------
+// Bound by the arcs' 4 bytes and the depth gathers.  A warp takes 32 vertices and
+// deals their lists, laid end to end, to its lanes, four arcs each with the loads
+// issued together; the best neighbour of each vertex is kept by a shared-memory
+// minimum, which starts from the parent the search found (any of them is one level
+// up), so an arc to a larger id is dropped before its depth is gathered.  Lists of
+// more than kMinLong arcs are left as chunks to min_parent_long_kernel: a warp that
+// walked a hub's list by itself took 163 us at scale 16, where the search takes 60.
+constexpr int64_t kMinLong = 512;  // also the chunk length
+
+struct MinScratch {
+    int32_t incl[32];
+    uint32_t best[32];
+    int32_t up[32];  // depth of a parent
+    int64_t beg[32];
+};
+
+__global__ void __launch_bounds__(256) min_parent_kernel(const int64_t *off, const uint32_t *adj,
+                                                         int64_t n, const int32_t *depth,
+                                                         int64_t *parent, bool seeded, uint2 *chunks,
+                                                         unsigned long long *count)
 {
-    const int lane = threadIdx.x & 31;
+    __shared__ MinScratch scratch[8];
+    MinScratch &ws = scratch[threadIdx.x >> 5];
+    const int lane = lane_id();
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long words = (n + 31) / 32;
-    for (long long w = gw; w < words; w += nw) {
+    for (long long w = gw; w < (n + 31) / 32; w += nw) {
         const int64_t v = w * 32 + lane;
-        int32_t dv = v < n ? depth[v] : -1;
-        int64_t b = 0, e = 0;
-        uint32_t best = 0xFFFFFFFFu;
-        const bool want = dv > 0;
-        if (want) {
-            b = off[v];
-            e = off[v + 1];
-            if (e - b <= 32) {
-                for (int64_t k = b; k < e; ++k) {
-                    uint32_t u = adj[k];
-                    if (u < best && depth[u] == dv - 1) { best = u; }
+        const int32_t dv = v < n ? depth[v] : -1;
+        int64_t beg = 0, deg = 0;
+        uint32_t first = 0xFFFFFFFFu;
+        if (dv > 0) {
+            beg = off[v];
+            deg = off[v + 1] - beg;
+            if (seeded) { first = (uint32_t)parent[v]; }
+        }
+        const bool longer = deg > kMinLong;
+        if (longer && !seeded) { parent[v] = (int64_t)first; }
+        unsigned owners = __ballot_sync(kFull, longer);
+        while (owners) {
+            const int o = __ffs(owners) - 1;
+            owners &= owners - 1;
+            const long long k = (__shfl_sync(kFull, deg, o) + kMinLong - 1) / kMinLong;
+            unsigned long long at = 0;
+            if (lane == 0) { at = atomicAdd(count, (unsigned long long)k); }
+            at = __shfl_sync(kFull, at, 0);
+            for (long long i = lane; i < k; i += 32) {
+                chunks[at + i] = make_uint2((uint32_t)(w * 32 + o), (uint32_t)i);
+            }
+        }
+        const int32_t len = longer ? 0 : (int32_t)deg;
+        const int32_t incl = warp_incl_scan(len);
+        const int32_t total = __shfl_sync(kFull, incl, 31);
+        if (total == 0) { continue; }
+        ws.incl[lane] = incl;
+        ws.best[lane] = first;
+        ws.up[lane] = dv - 1;
+        ws.beg[lane] = beg;
+        __syncwarp();
+        for (int32_t base = 0; base < total; base += 32 * kILP) {
+            int at[kILP];
+            uint32_t u[kILP];
+            bool in[kILP];
+#pragma unroll
+            for (int i = 0; i < kILP; ++i) { at[i] = 0; }  // lists that end at or before arc e
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+#pragma unroll
+                for (int i = 0; i < kILP; ++i) {
+                    if (ws.incl[at[i] + d - 1] <= base + i * 32 + lane) { at[i] += d; }
                 }
             }
-        }
-        unsigned big = __ballot_sync(kFull, want && e - b > 32);
-        while (big) {
-            const int owner = __ffs(big) - 1;
-            big &= big - 1;
-            const int64_t bb = __shfl_sync(kFull, b, owner);
-            const int64_t ee = __shfl_sync(kFull, e, owner);
-            const int32_t d = __shfl_sync(kFull, dv, owner);
-            uint32_t mine = 0xFFFFFFFFu;
-            for (int64_t k = bb + lane; k < ee; k += 32) {
-                uint32_t u = adj[k];
-                if (u < mine && depth[u] == d - 1) { mine = u; }
+#pragma unroll
+            for (int i = 0; i < kILP; ++i) {
+                const int32_t e = base + i * 32 + lane;
+                in[i] = e < total;
+                u[i] = 0;
+                if (in[i]) {
+                    u[i] = __ldg(&adj[ws.beg[at[i]] + (e - (at[i] ? ws.incl[at[i] - 1] : 0))]);
+                }
+            }
+            int32_t du[kILP];
+#pragma unroll
+            for (int i = 0; i < kILP; ++i) {
+                in[i] = in[i] && u[i] < *(volatile uint32_t *)&ws.best[at[i]];
+                du[i] = in[i] ? __ldg(&depth[u[i]]) : 0;
             }
 #pragma unroll
-            for (int s = 16; s > 0; s >>= 1) { mine = min(mine, __shfl_xor_sync(kFull, mine, s)); }
-            if (lane == owner) { best = mine; }
+            for (int i = 0; i < kILP; ++i) {
+                if (in[i] && du[i] == ws.up[at[i]]) { atomicMin(&ws.best[at[i]], u[i]); }
+            }
         }
-        if (want) { parent[v] = (int64_t)best; }
+        __syncwarp();
+        const uint32_t best = ws.best[lane];
+        if (len > 0 && (!seeded || best != first)) { parent[v] = (int64_t)best; }
+        __syncwarp();
+    }
+}
+
+// The chunks min_parent_kernel listed, one per warp at a time.  The last block
+// clears the count for the next launch.
+__global__ void __launch_bounds__(256) min_parent_long_kernel(const int64_t *off,
+                                                              const uint32_t *adj,
+                                                              const int32_t *depth,
+                                                              int64_t *parent, const uint2 *chunks,
+                                                              unsigned long long *count)
+{
+    const int lane = lane_id();
+    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    const long long total = (long long)__ldcg(&count[0]);
+    for (long long c = gw; c < total; c += nw) {
+        const uint2 q = __ldg(&chunks[c]);
+        const int64_t b = __ldg(&off[q.x]) + (int64_t)q.y * kMinLong;
+        const int64_t e = min(__ldg(&off[q.x + 1]), b + kMinLong);
+        const int32_t up = __ldg(&depth[q.x]) - 1;
+        // chunks of the same vertex lower it meanwhile: any value is a bound
+        const uint32_t bound = (uint32_t)__ldcg(&parent[q.x]);
+        uint32_t best = bound;
+        for (int64_t base = b; base < e; base += 32 * kILP) {
+            uint32_t u[kILP];
+            int32_t du[kILP];
+#pragma unroll
+            for (int i = 0; i < kILP; ++i) {
+                const int64_t k = base + i * 32 + lane;
+                u[i] = k < e ? __ldg(&adj[k]) : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (int i = 0; i < kILP; ++i) { du[i] = u[i] < best ? __ldg(&depth[u[i]]) : -2; }
+#pragma unroll
+            for (int i = 0; i < kILP; ++i) {
+                if (du[i] == up && u[i] < best) { best = u[i]; }
+            }
+        }
+        best = __reduce_min_sync(kFull, best);
+        if (lane == 0 && best < bound) {
+            atomicMin(reinterpret_cast<long long *>(&parent[q.x]), (long long)best);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&count[1], 1ull) == gridDim.x - 1) {
+        count[0] = 0;
+        count[1] = 0;
     }
 }
 
@@ -1464,6 +1568,7 @@ struct bd_bfs {
     PolicyBlob *policy = nullptr;  // device copy, or null
     KernelChoice kernel{nullptr, 0, 0};
     int grid = 0;
+    MinParentScratch min_scratch;  // opts.min_parent
     bool ctrl_valid = false;  // no launch has failed since the control block was zeroed
     int64_t cap_large = 0;
     // BD_ORDER_HUB graphs: depths and parents in the caller's numbering,
@@ -1601,9 +1706,7 @@ bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t star
         }
         BD_CUDA(cudaGetLastError());
         if (b->opts.min_parent) {
-            min_parent_kernel<<<grid_for(bitmap_words(n) * 32), 256, 0, b->stream>>>(
-                b->g->d_off, b->g->d_adj, n, out_depth, out_parent);
-            BD_CUDA(cudaGetLastError());
+            BD_CUDA(launch_min_parent(b->g, b->min_scratch, out_depth, out_parent, b->stream));
         }
     } else if (b->opts.min_parent) {
         // the smallest parent in the caller's numbering: on a hub graph, map
@@ -1619,9 +1722,7 @@ bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t star
             depth = b->out_depth;
             parent = b->out_parent;
         }
-        min_parent_kernel<<<grid_for(bitmap_words(n) * 32), 256, 0, b->stream>>>(
-            b->g->d_off, b->g->d_adj, n, depth, parent);
-        BD_CUDA(cudaGetLastError());
+        BD_CUDA(launch_min_parent(b->g, b->min_scratch, depth, parent, b->stream));
     }
     if (stop) { BD_CUDA(cudaEventRecord(stop, b->stream)); }
     return BD_OK;
@@ -1712,6 +1813,7 @@ void bfs_free(bd_bfs *b)
     cudaFree(b->rec);
     cudaFree(b->d_sources);
     cudaFree(b->policy);
+    min_parent_free(&b->min_scratch);
     if (b->ev0) { cudaEventDestroy(b->ev0); }
     if (b->ev1) { cudaEventDestroy(b->ev1); }
     if (b->stream) { cudaStreamDestroy(b->stream); }
@@ -1720,10 +1822,32 @@ void bfs_free(bd_bfs *b)
 
 }  // namespace
 
-cudaError_t launch_min_parent(const int64_t *off, const uint32_t *adj, int64_t n,
-                              const int32_t *depth, int64_t *parent, cudaStream_t s)
+cudaError_t min_parent_alloc(const bd_graph *g, MinParentScratch *s)
 {
-    min_parent_kernel<<<grid_for(bitmap_words(n) * 32), 256, 0, s>>>(off, adj, n, depth, parent);
+    if (g->max_degree <= kMinLong) { return cudaSuccess; }  // nothing is ever listed
+    // a list of more than kMinLong arcs has less than 2 arcs / kMinLong chunks
+    cudaError_t e = cudaMalloc(&s->chunks, sizeof(uint2) * (2 * g->arcs / kMinLong));
+    if (e == cudaSuccess) { e = cudaMalloc(&s->count, sizeof(unsigned long long) * 2); }
+    if (e == cudaSuccess) { e = cudaMemset(s->count, 0, sizeof(unsigned long long) * 2); }
+    return e;
+}
+
+void min_parent_free(MinParentScratch *s)
+{
+    cudaFree(s->chunks);
+    cudaFree(s->count);
+    *s = MinParentScratch{};
+}
+
+cudaError_t launch_min_parent(const bd_graph *g, const MinParentScratch &s, const int32_t *depth,
+                              int64_t *parent, cudaStream_t stream)
+{
+    min_parent_kernel<<<grid_for(bitmap_words(g->n) * 32), 256, 0, stream>>>(
+        g->d_off, g->d_adj, g->n, depth, parent, g->symmetric, s.chunks, s.count);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || !s.chunks) { return e; }
+    min_parent_long_kernel<<<148 * 4, 256, 0, stream>>>(g->d_off, g->d_adj, depth, parent, s.chunks,
+                                                        s.count);
     return cudaGetLastError();
 }
 
@@ -1777,7 +1901,8 @@ bd_status bd_bfs_create(bd_graph *g, const bd_bfs_opts *opts, bd_bfs **out)
               (!g->d_perm || (cudaMalloc(&b->out_depth, sizeof(int32_t) * n) == cudaSuccess &&
                               cudaMalloc(&b->out_parent, sizeof(int64_t) * n) == cudaSuccess)) &&
               cudaMalloc(&b->ctrl, sizeof(Ctrl)) == cudaSuccess &&
-              cudaMalloc(&b->rec, sizeof(bd_step) * kRecCap) == cudaSuccess;
+              cudaMalloc(&b->rec, sizeof(bd_step) * kRecCap) == cudaSuccess &&
+              (!o.min_parent || min_parent_alloc(g, &b->min_scratch) == cudaSuccess);
     for (int i = 0; i < 2 && ok; ++i) {
         ok = cudaMalloc(&b->vis[i], sizeof(uint32_t) * words) == cudaSuccess &&
              cudaMalloc(&b->qs[i], sizeof(uint32_t) * n) == cudaSuccess &&

@@ -546,15 +546,25 @@ __global__ void degree_keys_kernel(const uint32_t *src, const uint32_t *adj, con
     }
 }
 
-__global__ void count_live_kernel(const int64_t *off, int64_t n, unsigned long long *live)
+// stats[0] += vertices of nonzero degree, stats[1] = max degree (both zero before).
+__global__ void degree_stats_kernel(const int64_t *off, int64_t n, unsigned long long *stats)
 {
-    unsigned long long c = 0;
+    unsigned long long c = 0, m = 0;
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
          v += (int64_t)gridDim.x * blockDim.x) {
-        c += off[v + 1] != off[v];
+        const unsigned long long d = (unsigned long long)(off[v + 1] - off[v]);
+        c += d != 0;
+        m = d > m ? d : m;
     }
-    for (int d = 16; d > 0; d >>= 1) { c += __shfl_xor_sync(0xFFFFFFFFu, c, d); }
-    if ((threadIdx.x & 31) == 0 && c) { atomicAdd(live, c); }
+    for (int d = 16; d > 0; d >>= 1) {
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, d);
+        const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, m, d);
+        m = o > m ? o : m;
+    }
+    if ((threadIdx.x & 31) == 0 && c) {
+        atomicAdd(&stats[0], c);
+        atomicMax(&stats[1], m);
+    }
 }
 
 __global__ void isolated_bitmap_kernel(const int64_t *off, int64_t n, uint32_t *bits)
@@ -856,15 +866,16 @@ bd_status graph_finish(bd_graph *g, cudaStream_t s)
     BD_CUDA(cudaMalloc(&g->d_isolated, sizeof(uint32_t) * (words ? words : 1)));
     isolated_bitmap_kernel<<<grid_for(words), kThreads, 0, s>>>(g->d_off, g->n, g->d_isolated);
     BD_CUDA(cudaGetLastError());
-    DevBuf<unsigned long long> live;
-    if (live.alloc(1) != cudaSuccess) { return BD_ERR_OOM; }
-    BD_CUDA(cudaMemsetAsync(live.p, 0, sizeof(unsigned long long), s));
-    count_live_kernel<<<grid_for(g->n), kThreads, 0, s>>>(g->d_off, g->n, live.p);
+    DevBuf<unsigned long long> stats;
+    if (stats.alloc(2) != cudaSuccess) { return BD_ERR_OOM; }
+    BD_CUDA(cudaMemsetAsync(stats.p, 0, sizeof(unsigned long long) * 2, s));
+    degree_stats_kernel<<<grid_for(g->n), kThreads, 0, s>>>(g->d_off, g->n, stats.p);
     BD_CUDA(cudaGetLastError());
-    unsigned long long nl = 0;
-    BD_CUDA(cudaMemcpyAsync(&nl, live.p, sizeof(nl), cudaMemcpyDeviceToHost, s));
+    unsigned long long got[2] = {0, 0};
+    BD_CUDA(cudaMemcpyAsync(got, stats.p, sizeof got, cudaMemcpyDeviceToHost, s));
     BD_CUDA(cudaStreamSynchronize(s));
-    g->n_live = (int64_t)nl;
+    g->n_live = (int64_t)got[0];
+    g->max_degree = (int64_t)got[1];
     return BD_OK;
 }
 

@@ -43,6 +43,7 @@ struct bd_graph {
     int64_t m = 0;          // undirected edges (arcs / 2)
     int64_t arcs = 0;       // entries of the adjacency array
     int64_t n_live = 0;     // vertices of nonzero degree
+    int64_t max_degree = 0;
     int32_t order = BD_ORDER_INSERTION;
     // Every arc u->v has its reverse v->u (graphs built from edge lists, and
     // unions of them); not assumed for a caller's CSR.
@@ -95,11 +96,20 @@ bd_status check_parents_device(const bd_graph *g, int64_t source, const int64_t 
 // has an arc to another label, or -1.
 bd_status check_components_device(const bd_graph *g, const int64_t *d_label, int32_t *ok,
                                   int64_t *bad_vertex);
-// The deterministic parent tree (bd_bfs.cu): for every vertex of depth
-// d > 0, the smallest neighbour of depth d - 1 in the CSR (off, adj), written
-// to parent; other entries are left as they are.  Queued on s.
-cudaError_t launch_min_parent(const int64_t *off, const uint32_t *adj, int64_t n,
-                              const int32_t *depth, int64_t *parent, cudaStream_t s);
+// The deterministic parent tree (bd_bfs.cu).  Its scratch belongs to a handle:
+// one launch at a time.
+struct MinParentScratch {
+    uint2 *chunks = nullptr;              // {vertex, chunk} of long lists
+    unsigned long long *count = nullptr;  // [0] chunks listed, [1] blocks done
+};
+cudaError_t min_parent_alloc(const bd_graph *g, MinParentScratch *s);
+void min_parent_free(MinParentScratch *s);
+// For every vertex of depth d > 0, the smallest neighbour of depth d - 1 in the
+// caller's CSR, written to parent (which holds some such neighbour already in
+// graphs known to be symmetric); other entries are left as they are.  Queued on
+// stream.
+cudaError_t launch_min_parent(const bd_graph *g, const MinParentScratch &s, const int32_t *depth,
+                              int64_t *parent, cudaStream_t stream);
 // BD_ORDER_HUB: builds the renumbered traversal CSR of a finished graph.
 bd_status graph_build_hub(bd_graph *g, cudaStream_t s);
 // Fills d_isolated from d_off.

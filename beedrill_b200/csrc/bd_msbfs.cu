@@ -1395,6 +1395,7 @@ struct bd_msbfs {
     std::vector<int64_t> sources;  // roots of the last run
     bool ran = false;
     PolicyBlob *policy = nullptr;  // device copy, or null
+    MinParentScratch min_scratch;  // opts.min_parent
     uint2 *dq = nullptr;  // chunks of long pull scans, or null: no list is that long
     cudaGraphExec_t graph = nullptr;
     int graph_count = -1;
@@ -1487,7 +1488,7 @@ bd_status ms_enqueue_materialize(bd_msbfs *b, int group, int count)
     if (b->opts.min_parent) {
         for (int r = 0; r < count; ++r) {
             const int64_t row = ((int64_t)group * 64 + r) * n;
-            BD_CUDA(launch_min_parent(b->g->d_off, b->g->d_adj, n, b->out_depth + row,
+            BD_CUDA(launch_min_parent(b->g, b->min_scratch, b->out_depth + row,
                                       b->out_parent + row, b->stream));
         }
     }
@@ -1593,6 +1594,7 @@ void ms_free(bd_msbfs *b)
     cudaFree(b->d_counts);
     cudaFree(b->policy);
     cudaFree(b->dq);
+    min_parent_free(&b->min_scratch);
     cudaFree(b->out_depth);
     cudaFree(b->out_parent);
     cudaFree(b->xbuf);
@@ -1728,6 +1730,7 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
               cudaMalloc(&b->rec, sizeof(bd_step) * kMsRecCap) == cudaSuccess &&
               cudaMalloc(&b->d_sources, sizeof(int64_t) * 64 * b->groups) == cudaSuccess &&
               cudaMalloc(&b->d_counts, sizeof(unsigned long long) * 128 * b->groups) == cudaSuccess;
+    ok = ok && (!o.min_parent || min_parent_alloc(g, &b->min_scratch) == cudaSuccess);
     for (int i = 0; i < 3 && ok; ++i) {
         ok = cudaMalloc(&b->F[i], sizeof(ull) * n) == cudaSuccess &&
              cudaMalloc(&b->qs[i], sizeof(uint32_t) * n) == cudaSuccess &&

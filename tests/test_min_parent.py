@@ -1,0 +1,46 @@
+"""The deterministic tree around the length at which a list is cut into chunks
+(512 arcs), on graphs known to be symmetric and on a caller's CSR."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+bd = pytest.importorskip("beedrill_b200")
+
+
+def _two_hubs(width):
+    """0 - (1..width) - last: the last vertex and 0 have `width` neighbours, ids
+    shuffled so that the smallest parent is nowhere in particular in a list."""
+    n = width + 2
+    rng = np.random.default_rng(width)
+    ids = rng.permutation(n)
+    mid = np.arange(1, width + 1)
+    src = np.concatenate([np.zeros(width, np.int64), mid])
+    dst = np.concatenate([mid, np.full(width, n - 1)])
+    order = rng.permutation(2 * width)
+    return n, ids[src][order], ids[dst][order], int(ids[0])
+
+
+@pytest.mark.parametrize("width", [1, 31, 32, 33, 511, 512, 513, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("form", ["edges", "hub", "csr"])
+def test_min_parent_around_the_chunk_length(width, form):
+    n, src, dst, root = _two_hubs(width)
+    g = bd.Graph.from_edges(n, src, dst, bd.ORDER_HUB if form == "hub" else bd.ORDER_INSERTION)
+    off, adj = g.csr()
+    if form == "csr":
+        g = bd.Graph.from_csr(off, adj)
+    depth = O.bfs_depth(off, adj, root)
+    want = O.min_parent(off, adj, root, depth)
+    single = bd.HybridBFS(g, min_parent=True)
+    for _ in range(2):
+        single.clear()
+        single.run(root)
+        assert np.array_equal(single.parents(), want)
+    ms = bd.BatchedBFS(g, 3, min_parent=True)
+    ms.run([root, root, int(src[0])])
+    for i, r in enumerate((root, root, int(src[0]))):
+        d = O.bfs_depth(off, adj, r)
+        assert np.array_equal(ms.depths(i), d)
+        assert np.array_equal(ms.parents(i), O.min_parent(off, adj, r, d))
