@@ -1569,6 +1569,7 @@ struct bd_bfs {
     KernelChoice kernel{nullptr, 0, 0};
     int grid = 0;
     MinParentScratch min_scratch;  // opts.min_parent
+    CheckScratch check;
     bool ctrl_valid = false;  // no launch has failed since the control block was zeroed
     int64_t cap_large = 0;
     // BD_ORDER_HUB graphs: depths and parents in the caller's numbering,
@@ -1814,6 +1815,7 @@ void bfs_free(bd_bfs *b)
     cudaFree(b->d_sources);
     cudaFree(b->policy);
     min_parent_free(&b->min_scratch);
+    check_free(&b->check);
     if (b->ev0) { cudaEventDestroy(b->ev0); }
     if (b->ev1) { cudaEventDestroy(b->ev1); }
     if (b->stream) { cudaStreamDestroy(b->stream); }
@@ -2105,7 +2107,7 @@ bd_status bd_bfs_check(bd_bfs *b, int64_t source, int32_t *ok)
     if (source < 0 || source >= b->g->n) { return BD_ERR_RANGE; }
     const int64_t *parent = nullptr;
     BD_TRY(bd_bfs_device_ptrs(b, nullptr, &parent));
-    return check_parents_device(b->g, source, parent, ok, nullptr);
+    return check_parents_device(b->g, source, parent, ok, nullptr, &b->check);
 }
 
 bd_status bd_bfs_get_steps(bd_bfs *b, bd_step *steps, int64_t capacity, int64_t *count)

@@ -84,12 +84,22 @@ struct PolicyBlob;
 // Host-side PolicyBlob from the ABI's arrays (bd_policy.cu).
 bd_status policy_blob(const float *params, const float *mean, const float *inv_std,
                       const float *lo, const float *hi, float margin, PolicyBlob *blob);
+// Device memory of a check (bd_check.cu); a handle that checks its own results
+// keeps one, filled by its first check.
+struct CheckCtl;
+struct CheckScratch {
+    int32_t *depth = nullptr;
+    uint32_t *qs[2] = {nullptr, nullptr}, *ql[2] = {nullptr, nullptr};
+    unsigned long long *cb[2] = {nullptr, nullptr};
+    CheckCtl *ctl = nullptr;
+};
+void check_free(CheckScratch *s);
 // hybrid_bfs::check on the device (bd_check.cu) for a parent array in
 // device memory, in the reference's encoding and the caller's vertex ids;
 // *ok = 1 when it passes, *bad_vertex (may be null) gets the lowest failing
-// vertex or -1.
+// vertex or -1.  scratch null: allocated and freed by the call.
 bd_status check_parents_device(const bd_graph *g, int64_t source, const int64_t *d_parent,
-                               int32_t *ok, int64_t *bad_vertex);
+                               int32_t *ok, int64_t *bad_vertex, CheckScratch *scratch);
 // components::check on the device (bd_check.cu) for labels in device
 // memory (int64[n]); *ok = 1 when it passes, *bad_vertex (may be null) gets
 // the lowest vertex that is unreached from its label's representative or

@@ -1396,6 +1396,7 @@ struct bd_msbfs {
     bool ran = false;
     PolicyBlob *policy = nullptr;  // device copy, or null
     MinParentScratch min_scratch;  // opts.min_parent
+    CheckScratch check;
     uint2 *dq = nullptr;  // chunks of long pull scans, or null: no list is that long
     cudaGraphExec_t graph = nullptr;
     int graph_count = -1;
@@ -1595,6 +1596,7 @@ void ms_free(bd_msbfs *b)
     cudaFree(b->policy);
     cudaFree(b->dq);
     min_parent_free(&b->min_scratch);
+    check_free(&b->check);
     cudaFree(b->out_depth);
     cudaFree(b->out_parent);
     cudaFree(b->xbuf);
@@ -1866,7 +1868,7 @@ bd_status bd_msbfs_check(bd_msbfs *b, int32_t root_index, int32_t *ok)
     BD_TRY(ms_root_device(b, root_index, false, &parent));
     BD_CUDA(cudaStreamSynchronize(b->stream));
     return check_parents_device(b->g, b->sources[root_index], static_cast<const int64_t *>(parent),
-                                ok, nullptr);
+                                ok, nullptr, &b->check);
 }
 
 // Borrowed device pointers to one root's materialized results.
