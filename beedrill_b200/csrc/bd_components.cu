@@ -23,13 +23,19 @@
 // Which arcs are joined (symmetric CSR, every edge stored both ways), after
 // Sutton, Ben-Nun and Barak, "Optimizing Parallel Graph Connectivity
 // Computation via Subgraph Sampling" (IPDPS 2018, "Afforest"):
-//   cc_sample_first_kernel, cc_sample_second_kernel
-//                         every vertex joins its first arc, then its
-//                         second, each round followed by pointing every
-//                         vertex at its root (cc_flatten_kernel);
-//   the largest tree      found by sampling kProbe vertices' roots;
+//   cc_hook_kernel        every vertex points at the smallest of itself and its
+//                         first kHookArcs neighbours (a plain store: smaller ids
+//                         cannot form a cycle), then at its root
+//                         (cc_flatten_kernel);
+//   cc_merge_kernel       for one more arc of every vertex, the larger of the two
+//                         roots is lowered to the smaller by an atomicMin that
+//                         nobody waits for.  Where several arcs lower one root the
+//                         smallest wins and the others are dropped: nothing here
+//                         has to join every sampled arc, because the walk below
+//                         joins all arcs of what is left outside;
+//   cc_probe_kernel       the largest tree, by a vote of kProbe vertices' roots;
 //   cc_walk_kernel        every vertex OUTSIDE that tree (its parent word
-//                         is not the tree's root) joins the rest of its
+//                         is not the tree's root) joins all of its
 //                         arcs.  An edge between the largest tree and
 //                         another vertex is stored at that other vertex
 //                         too, and is joined from there, so skipping the
@@ -40,14 +46,18 @@
 //                         deals every listed vertex's arcs over the grid in
 //                         one flat range (a binary search per chunk, the
 //                         chunk prefix from cc_heavy_chunks_kernel).
+// (Joining the sampled arcs properly, by finds and atomicCAS, is what the first
+// version did: whenever two large trees met, every vertex between them tried the
+// same root word.  On file-order RMAT graphs that was 330 to 390 us for scale 18,
+// where hooking, two rounds of merging and three flattenings take 33; 170 to 510 us
+// at scale 22, where they take 180.)
 //   cc_compress_kernel    labels (each vertex's root), sizes per label
 //                         (one atomic per distinct label of a warp) and the
 //                         count of roots.
 // A CSR that does not hold every edge both ways takes every arc of every
 // vertex instead (the same cc_walk_kernel / cc_heavy_kernel pair).
+
 #include <algorithm>
-#include <cstring>
-#include <vector>
 
 #include "bd_internal.h"
 
@@ -57,8 +67,10 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int64_t kHeavy = 4096;    // arcs above which a vertex is split over the grid
-constexpr int kSampleArcs = 2;      // arc positions joined before the rest of the lists
-constexpr int kProbe = 1024;        // vertices whose roots vote for the largest tree
+constexpr int kHookArcs = 4;        // arcs a vertex looks at for its first parent
+constexpr int kMergeRounds = 2;     // and a third where the probe asks for it
+constexpr int kProbeOutside = 4;    // probed vertices outside the largest tree that do
+constexpr int kProbe = 256;         // vertices whose roots vote for the largest tree (one block)
 constexpr int64_t kHeavyChunk = 1024;  // arcs per unit of the heavy pass
 
 int grid_for_warps(int64_t warps)
@@ -142,34 +154,71 @@ __global__ void cc_init_kernel(uint32_t *parent, int64_t n, int64_t *size)
     }
 }
 
-// First sampling round: every vertex joins its first arc.  Its second arc
-// (in the same 32-byte sector of the adjacency) is kept in `second` for the
-// next round, which then reads 4 coalesced bytes per vertex instead of two
-// offsets and a random adjacency sector again; a vertex with fewer than two
-// arcs keeps its own id (joining itself does nothing).
-__global__ void cc_sample_first_kernel(const int64_t *off, const uint32_t *adj, int64_t n,
-                                       uint32_t *parent, uint32_t *second)
+// Every vertex's first parent, the arc cc_merge_kernel takes, and sizes: the
+// smallest of the vertex and its first kHookArcs neighbours (they share a sector
+// or two); of the others the first, or the vertex itself if there is none.
+// Isolated vertices are components of one already.
+__global__ void cc_hook_kernel(const int64_t *off, const uint32_t *adj, int64_t n,
+                               uint32_t *parent, uint32_t *second, int64_t *size)
 {
-    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n;
-         u += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = off[u], e = off[u + 1];
-        uint32_t nxt = (uint32_t)u;
-        if (e > b) {
-            const uint32_t a0 = __ldg(&adj[b]);
-            if (e - b > 1) { nxt = __ldg(&adj[b + 1]); }
-            cc_join(parent, (uint32_t)u, a0);
-        }
-        __stcs(&second[u], nxt);
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t b = off[v], e = off[v + 1];
+        const uint32_t u = (uint32_t)v;
+        uint32_t a[kHookArcs], lo = u, other = u;
+#pragma unroll
+        for (int j = 0; j < kHookArcs; ++j) { a[j] = b + j < e ? __ldg(&adj[b + j]) : u; }
+#pragma unroll
+        for (int j = 0; j < kHookArcs; ++j) { lo = min(lo, a[j]); }
+#pragma unroll
+        for (int j = kHookArcs - 1; j >= 0; --j) { other = a[j] != lo && a[j] != u ? a[j] : other; }
+        parent[v] = lo;
+        __stcs(&second[v], other);
+        __stcs(&size[v], (int64_t)(b == e));
     }
 }
 
-// Second sampling round: every vertex joins its second arc.
-__global__ void cc_sample_second_kernel(const uint32_t *second, int64_t n, uint32_t *parent)
+// Every vertex points at its root.  A warp lowers each distinct larger root once,
+// and a block only to less than it has sent before (kSent roots, the first ones it
+// meets): the arcs between two large trees all lower the same word, and one L2
+// slice takes about one such request a nanosecond.  At scale 22 a request from
+// every warp took 155 us, of which 16 are the reads; hence also few, large blocks.
+constexpr int kMergeThreads = 1024;
+constexpr int kSent = 2048;
+__global__ void __launch_bounds__(kMergeThreads) cc_merge_kernel(const uint32_t *second, int64_t n,
+                                                                 uint32_t *parent,
+                                                                 const uint32_t *wanted)
 {
-    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n;
-         u += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = __ldcs(&second[u]);
-        if (v != (uint32_t)u) { cc_join(parent, (uint32_t)u, v); }
+    if (wanted && *wanted == 0) { return; }
+    __shared__ uint32_t key[kSent], sent[kSent];
+    for (int i = threadIdx.x; i < kSent; i += kMergeThreads) { key[i] = sent[i] = 0xffffffffu; }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; base < n;
+         base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t u = base + lane;
+        uint32_t hi = 0, lo = 0;
+        if (u < n) {
+            const uint32_t v = __ldcs(&second[u]);
+            // roots hooked meanwhile point elsewhere: that only changes which
+            // of the two trees' vertices is compared
+            const uint32_t ru = __ldca(&parent[u]), rv = v != (uint32_t)u ? __ldca(&parent[v]) : ru;
+            hi = max(ru, rv);
+            lo = min(ru, rv);
+        }
+        const bool want = hi != lo;
+        const unsigned live = __ballot_sync(0xffffffffu, want);
+        if (want) {
+            const unsigned same = __match_any_sync(live, hi);
+            const uint32_t least = __reduce_min_sync(same, lo);
+            if (lane == __ffs(same) - 1) {
+                const unsigned h = (hi * 2654435761u) >> 21;  // 11 bits: kSent
+                const uint32_t k = atomicCAS(&key[h], 0xffffffffu, hi);
+                if ((k != 0xffffffffu && k != hi) || least < atomicMin(&sent[h], least)) {
+                    atomicMin(&parent[hi], least);
+                }
+            }
+        }
     }
 }
 
@@ -177,8 +226,9 @@ __global__ void cc_sample_second_kernel(const uint32_t *second, int64_t n, uint3
 // written).  No join runs meanwhile, so the roots are fixed; the walks do
 // not split paths, so no thread moves a word another thread has already
 // pointed at its root.
-__global__ void cc_flatten_kernel(uint32_t *parent, int64_t n)
+__global__ void cc_flatten_kernel(uint32_t *parent, int64_t n, const uint32_t *wanted)
 {
+    if (wanted && *wanted == 0) { return; }
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
          v += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t p = __ldcg(&parent[v]);
@@ -187,27 +237,56 @@ __global__ void cc_flatten_kernel(uint32_t *parent, int64_t n)
     }
 }
 
-// Roots of kProbe vertices spread evenly over the ids.
-__global__ void cc_probe_kernel(uint32_t *parent, int64_t n, uint32_t *out)
+// giant[0]: the most frequent root of kProbe vertices spread evenly over the ids
+// (the smallest of equally frequent ones).  giant[1]: whether another merging round
+// pays, because kProbeOutside of them have neighbours but lie outside that tree (a
+// second large tree is left now and then; the walk would then read all its arcs:
+// scale 22 in file order 373 us without the third round, 278 with it, where other
+// graphs lose 20 to 75 us by a round they do not need).  One block, so that the
+// host need not look.
+__global__ void __launch_bounds__(kProbe) cc_probe_kernel(const uint32_t *parent, int64_t n,
+                                                          const uint32_t *isolated, uint32_t *giant,
+                                                          const uint32_t *wanted)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kProbe) {
-        const uint32_t v = (uint32_t)(((uint64_t)i * (uint64_t)n) / kProbe);
-        out[i] = cc_find(parent, v);
+    if (wanted && *wanted == 0) { return; }
+    __shared__ __align__(16) uint32_t root[kProbe];
+    __shared__ unsigned long long best[kProbe / 32];
+    const uint32_t v = (uint32_t)(((uint64_t)threadIdx.x * (uint64_t)n) / kProbe);
+    const uint32_t mine = cc_root(parent, v);
+    const bool lone = (isolated[v >> 5] >> (v & 31)) & 1u;
+    root[threadIdx.x] = mine;
+    __syncthreads();
+    unsigned votes = 0;
+    const uint4 *r4 = reinterpret_cast<const uint4 *>(root);
+#pragma unroll 8
+    for (int i = 0; i < kProbe / 4; ++i) {
+        const uint4 r = r4[i];
+        votes += (r.x == mine) + (r.y == mine) + (r.z == mine) + (r.w == mine);
+    }
+    const unsigned top = __reduce_max_sync(0xffffffffu, votes);
+    const uint32_t who = __reduce_min_sync(0xffffffffu, votes == top ? mine : 0xffffffffu);
+    if ((threadIdx.x & 31) == 0) { best[threadIdx.x >> 5] = ((unsigned long long)top << 32) | ~who; }
+    __syncthreads();
+    unsigned long long m = 0;
+    for (int i = 0; i < kProbe / 32; ++i) { m = best[i] > m ? best[i] : m; }
+    const uint32_t g = ~(uint32_t)m;
+    const int outside = __syncthreads_count(mine != g && !lone);
+    if (threadIdx.x == 0) {
+        giant[0] = g;
+        giant[1] = outside >= kProbeOutside;
     }
 }
 
-// Arcs [first, e) of the vertices of a warp's 32-vertex group that have
+// The arcs of the vertices of a warp's 32-vertex group that have
 // work: each such vertex's list is walked by the whole warp, 32 arcs a
 // round; lists longer than kHeavy are appended to `heavy` instead.
-// skip_root: vertices whose root is this id have no work (the largest
-// tree), or ~0u for none; first: arc position to start at; all_arcs: join
-// every arc (else only arcs to smaller ids: each edge once, from its larger
-// endpoint).
+// giant: vertices whose root is this id have no work (the largest tree); null:
+// every vertex has.
 __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
-    const int64_t *off, const uint32_t *adj, int64_t n, uint32_t *parent, uint32_t skip_root,
-    int first, int all_arcs, uint32_t *heavy, unsigned long long *heavy_count)
+    const int64_t *off, const uint32_t *adj, int64_t n, uint32_t *parent, const uint32_t *giant,
+    uint32_t *heavy, unsigned long long *heavy_count)
 {
+    const uint32_t skip_root = giant ? *giant : 0u;
     const int lane = threadIdx.x & 31;
     const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -216,9 +295,12 @@ __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
         int64_t b = 0, e = 0;
         bool work = false;
         if (u < n) {
-            b = off[u] + first;
-            e = off[u + 1];
-            work = b < e && (skip_root == ~0u || __ldcg(&parent[u]) != skip_root);
+            work = !giant || __ldcg(&parent[u]) != skip_root;
+            if (work) {
+                b = off[u];
+                e = off[u + 1];
+                work = b < e;
+            }
             if (work && e - b > kHeavy) {
                 heavy[atomicAdd(heavy_count, 1ull)] = (uint32_t)u;
                 work = false;
@@ -232,8 +314,7 @@ __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
             const int64_t ee = __shfl_sync(0xffffffffu, e, owner);
             const uint32_t uu = (uint32_t)(base + owner);
             for (int64_t k = bb + lane; k < ee; k += 32) {
-                const uint32_t v = __ldg(&adj[k]);
-                if (all_arcs || v < uu) { cc_join(parent, uu, v); }
+                cc_join(parent, uu, __ldg(&adj[k]));
             }
         }
     }
@@ -242,7 +323,7 @@ __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
 // Chunk prefix of the heavy list: cbase[i] = chunks of heavy vertices < i.
 // One block of 1024 threads scans 1024 entries per round.
 __global__ void __launch_bounds__(1024) cc_heavy_chunks_kernel(
-    const int64_t *off, const uint32_t *heavy, const unsigned long long *heavy_count, int first,
+    const int64_t *off, const uint32_t *heavy, const unsigned long long *heavy_count,
     unsigned long long *cbase)
 {
     __shared__ unsigned long long warp_tot[32];
@@ -256,7 +337,7 @@ __global__ void __launch_bounds__(1024) cc_heavy_chunks_kernel(
         unsigned long long c = 0;
         if (i < count) {
             const uint32_t u = heavy[i];
-            const int64_t len = off[u + 1] - (off[u] + first);
+            const int64_t len = off[u + 1] - off[u];
             c = (unsigned long long)((len + kHeavyChunk - 1) / kHeavyChunk);
         }
         unsigned long long incl = c;
@@ -289,8 +370,7 @@ __global__ void __launch_bounds__(1024) cc_heavy_chunks_kernel(
 // vertex), so no thread walks one vertex's chunks after another.
 __global__ void __launch_bounds__(kThreads) cc_heavy_kernel(
     const int64_t *off, const uint32_t *adj, uint32_t *parent, const uint32_t *heavy,
-    const unsigned long long *heavy_count, const unsigned long long *cbase, int first,
-    int all_arcs)
+    const unsigned long long *heavy_count, const unsigned long long *cbase)
 {
     const int lane = threadIdx.x & 31;
     const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -305,30 +385,31 @@ __global__ void __launch_bounds__(kThreads) cc_heavy_kernel(
             if ((int64_t)cbase[mid] <= c) { lo = mid; } else { hi = mid - 1; }
         }
         const uint32_t u = heavy[lo];
-        const int64_t b = off[u] + first + (c - (int64_t)cbase[lo]) * kHeavyChunk;
+        const int64_t b = off[u] + (c - (int64_t)cbase[lo]) * kHeavyChunk;
         const int64_t e = min(off[u + 1], b + kHeavyChunk);
         for (int64_t k = b + lane; k < e; k += 32) {
-            const uint32_t v = __ldg(&adj[k]);
-            if (all_arcs || v < u) { cc_join(parent, u, v); }
+            cc_join(parent, u, __ldg(&adj[k]));
         }
     }
 }
 
-// Labels, sizes and roots.  `hint` is a vertex of the largest tree (or
-// ~0u): the lanes whose label is that tree's root count it in a block-wide
+// Labels, sizes and roots.  `hint` is a vertex of the largest tree (or null):
+// the lanes whose label is that tree's root count it in a block-wide
 // total added once per block, as do the roots; the lanes of a warp that
-// share any other label add it once (__match_any_sync).  (One atomic per
+// share any other label add it once (__match_any_sync).  Isolated vertices, with
+// `isolated` given, have their size already.  (One atomic per
 // warp on the largest component's size and on the root count put a few
 // hundred thousand atomics on two addresses, which serialise at their L2
 // slices.)
-__global__ void cc_compress_kernel(uint32_t *parent, int64_t n, uint32_t hint, int64_t *label,
-                                   int64_t *size, unsigned long long *roots)
+__global__ void cc_compress_kernel(uint32_t *parent, int64_t n, const uint32_t *hint,
+                                   const uint32_t *isolated, int64_t *label, int64_t *size,
+                                   unsigned long long *roots)
 {
     __shared__ uint32_t giant;
     __shared__ unsigned long long blk_giant, blk_roots;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        giant = hint < n ? cc_root(parent, hint) : 0xFFFFFFFFu;
+        giant = hint ? cc_root(parent, *hint) : 0xFFFFFFFFu;
         blk_giant = blk_roots = 0;
     }
     __syncthreads();
@@ -345,13 +426,14 @@ __global__ void cc_compress_kernel(uint32_t *parent, int64_t n, uint32_t hint, i
             r = p == g ? g : cc_root(parent, p);
             __stcs(&label[v], (int64_t)r);
         }
-        const bool other = valid && r != g;
+        const bool alone = valid && isolated && (__ldg(&isolated[v >> 5]) >> lane) & 1u;
+        const bool other = valid && r != g && !alone;
         const unsigned same = __match_any_sync(0xffffffffu, other ? r : 0xFFFFFFFFu);
         if (other && lane == __ffs(same) - 1) {
             atomicAdd(reinterpret_cast<unsigned long long *>(&size[r]),
                       (unsigned long long)__popc(same));
         }
-        my_giant += (valid && r == g) ? 1ull : 0ull;
+        my_giant += (valid && r == g && !alone) ? 1ull : 0ull;
         my_roots += (valid && r == (uint32_t)v) ? 1ull : 0ull;
     }
     my_giant = warp_sum_u64(my_giant);
@@ -389,7 +471,7 @@ struct bd_components {
     uint32_t *parent = nullptr;            // [n] union-find forest
     uint32_t *heavy = nullptr;             // [arcs / kHeavy + 1] vertices split over the grid
     unsigned long long *cbase = nullptr;   // [arcs / kHeavy + 2] their chunk prefix
-    uint32_t *probe = nullptr;             // [kProbe] sampled roots
+    uint32_t *giant = nullptr;             // [0] root of the largest tree, [1] merge again
     unsigned long long *counters = nullptr;  // [0] heavy vertices, [1] roots
     int64_t *label = nullptr;              // [n] component_ (components.h:13)
     int64_t *size = nullptr;               // [n] component_size_ (components.h:15)
@@ -407,7 +489,7 @@ void components_free(bd_components *c)
     cudaFree(c->parent);
     cudaFree(c->heavy);
     cudaFree(c->cbase);
-    cudaFree(c->probe);
+    cudaFree(c->giant);
     cudaFree(c->counters);
     cudaFree(c->label);
     cudaFree(c->size);
@@ -436,7 +518,7 @@ bd_status bd_components_create(bd_graph *g, bd_components **out)
         cudaMalloc(&c->parent, sizeof(uint32_t) * (n ? n : 1)) != cudaSuccess ||
         cudaMalloc(&c->heavy, sizeof(uint32_t) * heavy_cap) != cudaSuccess ||
         cudaMalloc(&c->cbase, sizeof(unsigned long long) * (heavy_cap + 1)) != cudaSuccess ||
-        cudaMalloc(&c->probe, sizeof(uint32_t) * bd::kProbe) != cudaSuccess ||
+        cudaMalloc(&c->giant, sizeof(uint32_t) * 2) != cudaSuccess ||
         cudaMalloc(&c->counters, sizeof(unsigned long long) * 2) != cudaSuccess ||
         cudaMalloc(&c->label, sizeof(int64_t) * (n ? n : 1)) != cudaSuccess ||
         cudaMalloc(&c->size, sizeof(int64_t) * (n ? n : 1)) != cudaSuccess) {
@@ -463,50 +545,39 @@ bd_status bd_components_run(bd_components *c, bd_components_stats *stats)
     cudaStream_t s = c->stream;
     BD_CUDA(cudaEventRecord(c->ev0, s));
     BD_CUDA(cudaMemsetAsync(c->counters, 0, sizeof(unsigned long long) * 2, s));
-    bd::cc_init_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, c->size);
-    uint32_t skip = ~0u;
-    int first = 0;
+    const uint32_t *giant = nullptr, *isolated = nullptr;
     if (g->symmetric) {
-        // the first and the second arc of every vertex, each round followed
-        // by pointing every vertex at its root (the next round's finds are
-        // short, and after the last one the largest tree's vertices are
-        // recognised by one parent word)
         // (the label array, written only by the final pass, holds the
-        // second arcs meanwhile)
+        // arcs to merge meanwhile)
         uint32_t *second = reinterpret_cast<uint32_t *>(c->label);
-        bd::cc_sample_first_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(
-            g->d_off, g->d_adj, n, c->parent, second);
-        bd::cc_flatten_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n);
-        bd::cc_sample_second_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(second, n, c->parent);
-        bd::cc_flatten_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n);
-        bd::cc_probe_kernel<<<(bd::kProbe + 255) / 256, 256, 0, s>>>(c->parent, n, c->probe);
-        BD_CUDA(cudaGetLastError());
-        std::vector<uint32_t> probe(bd::kProbe);
-        BD_CUDA(cudaMemcpyAsync(probe.data(), c->probe, sizeof(uint32_t) * bd::kProbe,
-                                cudaMemcpyDeviceToHost, s));
-        BD_CUDA(cudaStreamSynchronize(s));
-        // the most frequent root among the probes: the largest tree
-        std::sort(probe.begin(), probe.end());
-        size_t best = 0;
-        for (size_t i = 0, j = 0; i < probe.size(); i = j) {
-            for (j = i; j < probe.size() && probe[j] == probe[i]; ++j) {}
-            if (j - i > best) {
-                best = j - i;
-                skip = probe[i];
+        bd::cc_hook_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(g->d_off, g->d_adj, n, c->parent,
+                                                                    second, c->size);
+        bd::cc_flatten_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, nullptr);
+        const int merge_grid = std::min(bd::grid_for(n) / 4 + 1, 148 * 2);
+        const uint32_t *wanted = nullptr;  // the last round's kernels ask the probe
+        for (int round = 0; round <= bd::kMergeRounds; ++round) {
+            bd::cc_merge_kernel<<<merge_grid, bd::kMergeThreads, 0, s>>>(second, n, c->parent, wanted);
+            bd::cc_flatten_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, wanted);
+            if (round + 1 >= bd::kMergeRounds) {
+                bd::cc_probe_kernel<<<1, bd::kProbe, 0, s>>>(c->parent, n, g->d_isolated, c->giant,
+                                                             wanted);
+                wanted = c->giant + 1;
             }
         }
-        first = bd::kSampleArcs;
+        giant = c->giant;
+        isolated = g->d_isolated;
+    } else {
+        bd::cc_init_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, c->size);
     }
-    // symmetric: the rest of the arcs of vertices outside the largest tree;
+    // symmetric: the arcs of vertices outside the largest tree;
     // otherwise every arc of every vertex
     bd::cc_walk_kernel<<<bd::grid_for_warps(n), bd::kThreads, 0, s>>>(
-        g->d_off, g->d_adj, n, c->parent, skip, first, 1, c->heavy, c->counters);
-    bd::cc_heavy_chunks_kernel<<<1, 1024, 0, s>>>(g->d_off, c->heavy, c->counters, first,
-                                                  c->cbase);
+        g->d_off, g->d_adj, n, c->parent, giant, c->heavy, c->counters);
+    bd::cc_heavy_chunks_kernel<<<1, 1024, 0, s>>>(g->d_off, c->heavy, c->counters, c->cbase);
     bd::cc_heavy_kernel<<<148 * 8, bd::kThreads, 0, s>>>(g->d_off, g->d_adj, c->parent, c->heavy,
-                                                        c->counters, c->cbase, first, 1);
-    bd::cc_compress_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, skip, c->label,
-                                                                    c->size, c->counters + 1);
+                                                        c->counters, c->cbase);
+    bd::cc_compress_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(
+        c->parent, n, giant, isolated, c->label, c->size, c->counters + 1);
     BD_CUDA(cudaGetLastError());
     BD_CUDA(cudaEventRecord(c->ev1, s));
     unsigned long long roots = 0;
