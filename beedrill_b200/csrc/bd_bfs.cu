@@ -874,12 +874,15 @@ __device__ void end_step(const BfsParams &p, const StepView &sv, SharedState<BLO
         atomicMax(&acc->t_end, (unsigned long long)globaltimer());
         LevelState &st = sh.st;
         if (arrive_wait(p, sv.barrier, false)) {
-            Acc a;
-            a.found = __ldcg(&acc->found);
-            a.degsum = __ldcg(&acc->degsum);
-            a.small_cnt = __ldcg(&acc->small_cnt);
-            a.large_packed = __ldcg(&acc->large_packed);
+            // 16 bytes a request: all CTAs read this one line at once
+            const ulonglong2 *from = reinterpret_cast<const ulonglong2 *>(acc);
+            const ulonglong2 w0 = __ldcg(&from[0]), w1 = __ldcg(&from[1]);
             const long long t_end = (long long)__ldcg(&acc->t_end);
+            Acc a;
+            a.found = w0.x;
+            a.degsum = w0.y;
+            a.small_cnt = w1.x;
+            a.large_packed = w1.y;
             if (blockIdx.x == 0) { record_step(p, st, (long long)a.found, t_end); }
             advance(st, p, a, t_end);
         } else {
@@ -1195,7 +1198,11 @@ __device__ __noinline__ void solo_run(bool init)
             q ^= 1;
             shared_queue = true;
         } else {
-            if (threadIdx.x == 0) { sh.queued = 0; }
+            if (threadIdx.x == 0) {
+                sh.queued = 0;
+                sh.acc.small_cnt = sh.acc.large_packed = 0;
+            }
+            __syncthreads();
             const StepView sv = view_of(sh.st);
             const Team team{(long long)(threadIdx.x >> 5), BLOCK / 32, &sh.acc};
             bu_step<BLOCK, 1>(p, sv, team, loc);
@@ -1214,8 +1221,10 @@ __device__ __noinline__ void solo_run(bool init)
             record_step(p, st, (long long)tf, t_end);
             advance(st, p, a, t_end);
             decide_rule(st, p, sh.rule_dir, sh.consult);
-            // what lies in the global queues counts for this frontier only
-            if (!shared_queue || solo_applies<BLOCK>(st, p)) {
+            // what lies in the global queues counts for this frontier only (the
+            // policy may still change the direction, not the size: past the
+            // shared queue a top-down level is the grid's either way)
+            if (!shared_queue || st.f_count <= kSoloCap<BLOCK>) {
                 sh.acc.small_cnt = sh.acc.large_packed = 0;
             }
         }

@@ -35,7 +35,7 @@ constexpr unsigned long long kChunkMask = (1ull << kLargeShift) - 1;
 // (b + 1) % 3 before it arrives there (every CTA finished reading it before
 // arriving at barrier b - 1).  Barriers are numbered through from launch to
 // launch, so a launch finds its first slot clear.
-struct Acc {
+struct alignas(16) Acc {
     unsigned long long found;
     unsigned long long degsum;
     unsigned long long small_cnt;
@@ -72,7 +72,7 @@ struct LevelState {
 };
 
 // Device-resident control block of one BFS handle.
-struct Ctrl {
+struct alignas(16) Ctrl {
     unsigned long long bar;      // arrivals; barrier b is complete at (b + 1) * CTAs
     int error;
     int pad0;

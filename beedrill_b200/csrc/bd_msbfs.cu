@@ -59,7 +59,7 @@ constexpr unsigned kRecSlots = 16;  // delivery records per vertex
 
 // Counters of one step, in a ring of three slots (step s uses s % 3; CTA 0
 // clears (s + 1) % 3 during step s, after every CTA has read it).
-struct MsAcc {
+struct alignas(16) MsAcc {
     ull vertices;    // vertices entering the next frontier
     ull degsum;      // their degree sum
     ull lanes;       // new (vertex, lane) pairs
@@ -67,8 +67,8 @@ struct MsAcc {
     ull large_packed;
     ull done_degsum; // degree sum of vertices that just got every lane
     ull t_end;       // max over CTAs of their arrival time
-    ull work;        // pull steps: next bitmap word to hand out
     ull lanes_or;    // lanes delivered in the step (the next frontier's lanes)
+    ull work;        // pull steps: next bitmap word to hand out
     ull deferred;    // pull steps: chunks of long lists left for all warps
 };
 
@@ -767,7 +767,7 @@ struct MsShared {
     ull red[5][BLOCK / 32];
     MsState st;     // this CTA's copy of the state
     PolicyBlob pol; // the learned policy's weights, staged once
-    int rule_dir;
+    int consult;    // the policy decides the next step
     bool listed;    // pull step: all chunks of long lists are on dq
 };
 
@@ -803,37 +803,6 @@ __device__ void ms_advance(MsState &c, const MsAcc &a, long long t_end)
     if (c.dir == kPush) { c.push_steps += 1; } else { c.pull_steps += 1; }
     c.level += 1;
     c.step += 1;
-}
-
-// Next direction: the rule, or the learned policy (warp 0, weights from w)
-// where it is installed, trusted and confident.  Every thread of the block.
-template <typename Shared>
-__device__ void ms_decide(MsState &c, const MsParams &p, const PolicyBlob *w, Shared &sh)
-{
-    const int tid = threadIdx.x;
-    if (tid == 0) { sh.rule_dir = ms_rule(c, p); }
-    __syncthreads();
-    // the network runs only where the frontier's degree sum over the
-    // unexplored one lies in the band the policy was trained to decide in
-    const bool learned = p.policy && p.force_dir < 0 && sh.rule_dir != kMsDone &&
-                         policy_in_band(w, c.f_degsum, c.arcs_left);
-    if (!learned) {
-        if (tid == 0) { c.dir = sh.rule_dir; }
-        return;
-    }
-    if (tid < 32) {
-        const float gap = policy_gap_warp(w, c.f_count, c.f_degsum, c.arcs_left, c.level, p.n,
-                                          p.m, c.prev_dir, c.prev_ns);
-        if (tid == 0) {
-            int d = sh.rule_dir;
-            if (isfinite(gap) && fabsf(gap) >= w->margin) {
-                const int pick = gap > 0.f ? kPull : kPush;
-                if (pick != d) { c.policy_overrides += 1; }
-                d = pick;
-            }
-            c.dir = d;
-        }
-    }
 }
 
 // The end of a step: block reduction of the counters, arrival at the grid
@@ -879,15 +848,19 @@ __device__ void ms_end_step(const MsParams &p, const MsView &sv, MsShared<BLOCK>
         const bool ok = ms_arrive_wait(p, st.bars);
         st.bars += 1;
         if (ok && __ldcg(&c->error) == 0) {
+            // 16 bytes a request: all CTAs read this one line at once
+            const ulonglong2 *from = reinterpret_cast<const ulonglong2 *>(acc);
+            const ulonglong2 w0 = __ldcg(&from[0]), w1 = __ldcg(&from[1]), w2 = __ldcg(&from[2]),
+                             w3 = __ldcg(&from[3]);
             MsAcc a;
-            a.vertices = __ldcg(&acc->vertices);
-            a.degsum = __ldcg(&acc->degsum);
-            a.lanes = __ldcg(&acc->lanes);
-            a.small_cnt = __ldcg(&acc->small_cnt);
-            a.large_packed = __ldcg(&acc->large_packed);
-            a.done_degsum = __ldcg(&acc->done_degsum);
-            a.lanes_or = __ldcg(&acc->lanes_or);
-            const long long t_end = (long long)__ldcg(&acc->t_end);
+            a.vertices = w0.x;
+            a.degsum = w0.y;
+            a.lanes = w1.x;
+            a.small_cnt = w1.y;
+            a.large_packed = w2.x;
+            a.done_degsum = w2.y;
+            a.lanes_or = w3.y;
+            const long long t_end = (long long)w3.x;
             if (s == 0) { st.t_last = (long long)__ldcg(&c->t_start); }
             if (blockIdx.x == 0 && s < p.rec_cap) {
                 bd_step r;
@@ -904,10 +877,26 @@ __device__ void ms_end_step(const MsParams &p, const MsView &sv, MsShared<BLOCK>
         } else {
             st.f_count = 0;  // leave the loop
         }
+        st.dir = ms_rule(st, p);
+        // the network runs only where the frontier's degree sum over the
+        // unexplored one lies in the band the policy was trained to decide in
+        sh.consult = p.policy && p.force_dir < 0 && st.dir != kMsDone &&
+                     policy_in_band(&sh.pol, st.f_degsum, st.arcs_left);
     }
     __syncthreads();
-    ms_decide(sh.st, p, &sh.pol, sh);
-    __syncthreads();
+    if (sh.consult) {
+        if (threadIdx.x < 32) {
+            MsState &st = sh.st;
+            const float gap = policy_gap_warp(&sh.pol, st.f_count, st.f_degsum, st.arcs_left,
+                                              st.level, p.n, p.m, st.prev_dir, st.prev_ns);
+            if (threadIdx.x == 0 && isfinite(gap) && fabsf(gap) >= sh.pol.margin) {
+                const int pick = gap > 0.f ? kPull : kPush;
+                if (pick != st.dir) { st.policy_overrides += 1; }
+                st.dir = pick;
+            }
+        }
+        __syncthreads();
+    }
 }
 
 template <int BLOCK, int MINB>
