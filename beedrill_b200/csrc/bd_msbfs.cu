@@ -1159,9 +1159,9 @@ __global__ void ms_extract_kernel(const int32_t *depth, const uint32_t *parent, 
 // (root0 + r) gets depth_out[(root0 + r) * n + v] and parent_out[...] for
 // every caller vertex v (caller ids, the reference's encoding: the source is
 // its own parent, unreached vertices -deg or -1).  One pass over the group's
-// state instead of one per lane: thread i of a CTA takes caller vertex
-// v0 + i of a tile of kMatThreads consecutive vertices and
-//   fill   reads the vertex's seen word, record count and records once (a
+// state instead of one per lane: a thread takes V consecutive caller vertices
+// (two where the rows allow 16-byte stores, n even, else one) and
+//   fill   reads each vertex's seen word, record count and records once (a
 //          record covers every lane one provider delivered at one level, so
 //          the provider is renamed once per record) and the per-lane rows of
 //          lanes past its records.  Every distinct (depth, parent) pair gets
@@ -1171,13 +1171,18 @@ __global__ void ms_extract_kernel(const int32_t *depth, const uint32_t *parent, 
 //          of lane r's slot): a record sets its lanes in four ORs, whatever
 //          their number, so the threads of a warp do not wait for the one
 //          whose records hold the most lanes;
-//   write  walks the roots with the planes shifted one lane a step: the
-//          lane's slot gives its depth and parent with no branch, and the
-//          CTA's threads store each root's row entries for kMatThreads
-//          consecutive vertices, streaming past L2.
+//   write  walks the roots eight at a time: a byte of each plane becomes eight
+//          4-bit slots, a slot gives a lane's depth and parent with no branch,
+//          and the CTA's threads store each root's row entries of consecutive
+//          vertices, streaming past L2.
 // No thread reads another's table, so there is no barrier and a warp's
 // writes overlap another's loads.  A lane whose pair finds the table full
 // reads its row in the write loop (more than 16 distinct deliverers).
+//
+// The bytes are 12 x 64 per vertex written and some 190 read in random sectors,
+// but one vertex per thread with the planes shifted lane by lane cost 55
+// instructions per (vertex, root) and was bound by issue and latency (scale 21:
+// 490 us, DRAM at 47 %).
 struct MsOutParams {
     const int32_t *depth;     // per-lane rows [n][R]
     const uint32_t *parent;
@@ -1194,10 +1199,7 @@ struct MsOutParams {
     int64_t *parent_out;
 };
 
-constexpr int kMatThreads = 256;
 constexpr unsigned kMatSlots = 16;
-// per thread: a (depth, parent) pair per slot, slot-major [kMatSlots][threads]
-constexpr size_t kMatSmem = (size_t)kMatThreads * kMatSlots * sizeof(uint2);
 
 // Adds `lanes` to the planes of slot k.
 __device__ __forceinline__ void mat_set_slot(ull (&plane)[4], unsigned k, ull lanes)
@@ -1206,123 +1208,191 @@ __device__ __forceinline__ void mat_set_slot(ull (&plane)[4], unsigned k, ull la
     for (int b = 0; b < 4; ++b) { plane[b] |= ((k >> b) & 1u) ? lanes : 0ull; }
 }
 
-__global__ void __launch_bounds__(kMatThreads) ms_materialize_kernel(MsOutParams o)
+__device__ __forceinline__ uint32_t mat_rename(const MsOutParams &o, uint32_t provider)
 {
-    extern __shared__ __align__(16) unsigned char mat_raw[];
-    const int tid = threadIdx.x;
-    uint2 *tab = reinterpret_cast<uint2 *>(mat_raw);  // [kMatSlots][threads]: {depth, parent}
-    const ull all = o.lanes >= 64 ? ~0ull : ((1ull << o.lanes) - 1);
-    const long long tiles = (o.n + kMatThreads - 1) / kMatThreads;
-    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int64_t v = tile * kMatThreads + tid;
-        if (v >= o.n) { continue; }
-        const int64_t t = o.perm ? (int64_t)__ldg(&o.perm[v]) : v;
-        const int64_t deg = __ldg(&o.off[v + 1]) - __ldg(&o.off[v]);
-        const ull s = __ldcs(&o.seen[t]) & all;
-        ull plane[4] = {0ull, 0ull, 0ull, 0ull};
-        ull row_lanes = 0;  // lanes read from their rows in the write loop
-        if (s) {
-            const uint4 *rv = o.rec + t * kRecSlots;
-            // the first two slots are read together with the count (they lie
-            // in the vertex's record block whatever the count says)
-            const uint4 x0 = __ldcs(&rv[0]), x1 = __ldcs(&rv[1]);
-            const unsigned cnt = min(__ldcs(&o.rec_cnt[t]), kRecSlots);
-            ull left = s;
-            for (unsigned k0 = 0; k0 < cnt && left; k0 += 4) {
-                uint4 x[4];
+    // (a provider id out of range would only come from a broken record; it is
+    // passed through, not followed)
+    return o.iperm && provider < o.n ? __ldg(&o.iperm[provider]) : provider;
+}
+
+// The table entries and planes of a vertex reached by lanes s: records x0, x1 and
+// cnt are read already.  tab: the vertex's entry of slot 0, `stride` apart.
+__device__ __forceinline__ void mat_fill(const MsOutParams &o, int64_t t, ull s, uint4 x0, uint4 x1,
+                                         unsigned cnt, uint2 *tab, int stride, ull (&plane)[4],
+                                         ull &row_lanes)
+{
+    const uint4 *rv = o.rec + t * kRecSlots;
+    ull left = s;
+    for (unsigned k0 = 0; k0 < cnt && left; k0 += 4) {
+        uint4 x[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    x[j] = (k0 == 0 && j < 2) ? (j ? x1 : x0)
-                                              : (k0 + j < cnt ? __ldcs(&rv[k0 + j])
-                                                              : make_uint4(0, 0, 0, 0));
-                }
+        for (int j = 0; j < 4; ++j) {
+            x[j] = (k0 == 0 && j < 2) ? (j ? x1 : x0)
+                                      : (k0 + j < cnt ? __ldcs(&rv[k0 + j]) : make_uint4(0, 0, 0, 0));
+        }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const ull mask = k0 + j < cnt ? (((ull)x[j].y << 32) | x[j].x) & left : 0ull;
-                    if (!mask) { continue; }
-                    left &= ~mask;
-                    const unsigned k = k0 + j;
-                    // (a provider id out of range would only come from a
-                    // broken record; it is passed through, not followed)
-                    tab[k * kMatThreads + tid] = make_uint2(
-                        x[j].w, o.iperm && x[j].z < o.n ? __ldg(&o.iperm[x[j].z]) : x[j].z);
-                    mat_set_slot(plane, k, mask);
+        for (int j = 0; j < 4; ++j) {
+            const ull mask = k0 + j < cnt ? (((ull)x[j].y << 32) | x[j].x) & left : 0ull;
+            if (!mask) { continue; }
+            left &= ~mask;
+            const unsigned k = k0 + j;
+            tab[k * stride] = make_uint2(x[j].w, mat_rename(o, x[j].z));
+            mat_set_slot(plane, k, mask);
+        }
+    }
+    // lanes past the records: their rows, four loads in flight; lanes
+    // with the (depth, parent) pair of the previous one share its slot
+    unsigned used = cnt;
+    int32_t last_d = -2;
+    uint32_t last_p = 0;
+    unsigned last_k = kMatSlots;
+    while (left) {
+        int rr[4];
+        int32_t dd[4];
+        uint32_t pp[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            rr[j] = left ? __ffsll((long long)left) - 1 : -1;
+            left &= left ? left - 1 : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            dd[j] = rr[j] >= 0 ? __ldcs(&o.depth[t * o.R + rr[j]]) : 0;
+            pp[j] = rr[j] >= 0 ? __ldcs(&o.parent[t * o.R + rr[j]]) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (rr[j] < 0) { continue; }
+            if (dd[j] != last_d || pp[j] != last_p) {
+                last_d = dd[j];
+                last_p = pp[j];
+                last_k = kMatSlots;
+                if (used < kMatSlots) {
+                    last_k = used++;
+                    tab[last_k * stride] = make_uint2((uint32_t)dd[j], mat_rename(o, pp[j]));
                 }
             }
-            // lanes past the records: their rows, four loads in flight; lanes
-            // with the (depth, parent) pair of the previous one share its slot
-            unsigned used = cnt;
-            int32_t last_d = -2;
-            uint32_t last_p = 0;
-            unsigned last_k = kMatSlots;
-            while (left) {
-                int rr[4];
-                int32_t dd[4];
-                uint32_t pp[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    rr[j] = left ? __ffsll((long long)left) - 1 : -1;
-                    left &= left ? left - 1 : 0ull;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    dd[j] = rr[j] >= 0 ? __ldcs(&o.depth[t * o.R + rr[j]]) : 0;
-                    pp[j] = rr[j] >= 0 ? __ldcs(&o.parent[t * o.R + rr[j]]) : 0u;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (rr[j] < 0) { continue; }
-                    if (dd[j] != last_d || pp[j] != last_p) {
-                        last_d = dd[j];
-                        last_p = pp[j];
-                        last_k = kMatSlots;
-                        if (used < kMatSlots) {
-                            last_k = used++;
-                            tab[last_k * kMatThreads + tid] = make_uint2(
-                                (uint32_t)dd[j],
-                                o.iperm && pp[j] < o.n ? __ldg(&o.iperm[pp[j]]) : pp[j]);
-                        }
-                    }
-                    const ull bit = 1ull << rr[j];
-                    if (last_k < kMatSlots) {
-                        mat_set_slot(plane, last_k, bit);
-                    } else {
-                        row_lanes |= bit;
-                    }
-                }
+            const ull bit = 1ull << rr[j];
+            if (last_k < kMatSlots) {
+                mat_set_slot(plane, last_k, bit);
+            } else {
+                row_lanes |= bit;
             }
         }
-        const int64_t unreached = deg != 0 ? -deg : -1;
+    }
+}
+
+// Bits 0-7 of x to bits 0, 4, ... 28.
+__device__ __forceinline__ uint32_t mat_spread(uint32_t x)
+{
+    x &= 0xFFu;
+    x = (x | (x << 12)) & 0x000F000Fu;
+    x = (x | (x << 6)) & 0x03030303u;
+    return (x | (x << 3)) & 0x11111111u;
+}
+
+template <int V, int T>
+__global__ void __launch_bounds__(T) ms_materialize_kernel(MsOutParams o)
+{
+    static_assert(V == 1 || V == 2, "rows are stored one or two entries at a time");
+    extern __shared__ __align__(16) unsigned char mat_raw[];  // [kMatSlots][V][T] pairs
+    constexpr int stride = V * T;
+    uint2 *tab = reinterpret_cast<uint2 *>(mat_raw) + threadIdx.x;  // entry (k, i): [k * stride + i * T]
+    const ull all = o.lanes >= 64 ? ~0ull : ((1ull << o.lanes) - 1);
+    const long long tiles = (o.n + stride - 1) / stride;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t v = tile * stride + V * threadIdx.x;
+        if (v >= o.n) { continue; }  // V == 2: n is even
+        int64_t off[V + 1], t[V];
+        ull s[V];
+#pragma unroll
+        for (int i = 0; i <= V; ++i) { off[i] = __ldg(&o.off[v + i]); }
+#pragma unroll
+        for (int i = 0; i < V; ++i) { t[i] = o.perm ? (int64_t)__ldg(&o.perm[v + i]) : v + i; }
+#pragma unroll
+        for (int i = 0; i < V; ++i) { s[i] = __ldcs(&o.seen[t[i]]) & all; }
+        // the first two records are read together with the count (they lie
+        // in the vertex's record block whatever the count says)
+        uint4 x0[V], x1[V];
+        unsigned cnt[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            cnt[i] = 0;
+            x0[i] = x1[i] = make_uint4(0, 0, 0, 0);
+            if (s[i]) {
+                x0[i] = __ldcs(&o.rec[t[i] * kRecSlots]);
+                x1[i] = __ldcs(&o.rec[t[i] * kRecSlots + 1]);
+                cnt[i] = min(__ldcs(&o.rec_cnt[t[i]]), kRecSlots);
+            }
+        }
+        ull plane[V][4], row_lanes[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            row_lanes[i] = 0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) { plane[i][b] = 0; }
+            if (s[i]) {
+                mat_fill(o, t[i], s[i], x0[i], x1[i], cnt[i], tab + i * T, stride, plane[i],
+                         row_lanes[i]);
+            }
+        }
+        int64_t unreached[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const int64_t deg = off[i + 1] - off[i];
+            unreached[i] = deg != 0 ? -deg : -1;
+        }
         int32_t *dp = o.depth_out + v;
         int64_t *pq = o.parent_out + v;
-        // two halves of 32 lanes, so that the planes shift as 32-bit words
-        for (int h = 0; h < 2 && 32 * h < o.lanes; ++h) {
-            uint32_t g = (uint32_t)(s >> (32 * h)), rw = (uint32_t)(row_lanes >> (32 * h));
-            uint32_t q0 = (uint32_t)(plane[0] >> (32 * h)), q1 = (uint32_t)(plane[1] >> (32 * h));
-            uint32_t q2 = (uint32_t)(plane[2] >> (32 * h)), q3 = (uint32_t)(plane[3] >> (32 * h));
-            const int end = min(32, o.lanes - 32 * h);
-            for (int j = 0; j < end; ++j) {
-                const unsigned k = (q0 & 1u) | ((q1 & 1u) << 1) | ((q2 & 1u) << 2) | ((q3 & 1u) << 3);
-                const uint2 e = tab[k * kMatThreads + tid];
-                int32_t d = (int32_t)e.x;
-                int64_t par = (int64_t)e.y;
-                if (rw & 1u) {  // more pairs than slots: the lane's own row
-                    const int r = 32 * h + j;
-                    const uint32_t pr = __ldcs(&o.parent[t * o.R + r]);
-                    d = __ldcs(&o.depth[t * o.R + r]);
-                    par = (int64_t)(o.iperm && pr < o.n ? __ldg(&o.iperm[pr]) : pr);
+        for (int r0 = 0; r0 < o.lanes; r0 += 8) {
+            uint32_t slots[V], got[V];
+            uint32_t rows = 0;
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                slots[i] = mat_spread((uint32_t)plane[i][0]) | (mat_spread((uint32_t)plane[i][1]) << 1) |
+                           (mat_spread((uint32_t)plane[i][2]) << 2) |
+                           (mat_spread((uint32_t)plane[i][3]) << 3);
+                got[i] = (uint32_t)s[i] & 0xFFu;
+                rows |= (uint32_t)row_lanes[i] & 0xFFu;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                int32_t d[V];
+                int64_t par[V];
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    const uint2 e = tab[((slots[i] >> (4 * j)) & 15u) * stride + i * T];
+                    const bool has = (got[i] >> j) & 1u;
+                    d[i] = has ? (int32_t)e.x : -1;
+                    par[i] = has ? (int64_t)e.y : unreached[i];
                 }
-                const bool got = g & 1u;
-                __stcs(dp, got ? d : -1);
-                __stcs(pq, got ? par : unreached);
+                if ((rows >> j) & 1u) {  // more pairs than slots: the lane's own row
+#pragma unroll
+                    for (int i = 0; i < V; ++i) {
+                        if ((row_lanes[i] >> j) & 1ull) {
+                            d[i] = __ldcs(&o.depth[t[i] * o.R + r0 + j]);
+                            par[i] = (int64_t)mat_rename(o, __ldcs(&o.parent[t[i] * o.R + r0 + j]));
+                        }
+                    }
+                }
+                if (r0 + j < o.lanes) {
+                    if constexpr (V == 2) {
+                        __stcs(reinterpret_cast<int2 *>(dp), make_int2(d[0], d[1]));
+                        __stcs(reinterpret_cast<longlong2 *>(pq), make_longlong2(par[0], par[1]));
+                    } else {
+                        __stcs(dp, d[0]);
+                        __stcs(pq, par[0]);
+                    }
+                }
                 dp += o.n;
                 pq += o.n;
-                g >>= 1;
-                rw >>= 1;
-                q0 >>= 1;
-                q1 >>= 1;
-                q2 >>= 1;
-                q3 >>= 1;
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                s[i] >>= 8;
+                row_lanes[i] >>= 8;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) { plane[i][b] >>= 8; }
             }
         }
     }
@@ -1339,6 +1409,25 @@ __global__ void ms_long_chunks_kernel(const int64_t *off, int64_t n, int64_t lon
     }
     c = warp_sum(c);
     if (lane_id() == 0 && c) { atomicAdd(chunks, c); }
+}
+
+using MsRowsKernel = void (*)(MsOutParams);
+struct MsRows {
+    MsRowsKernel fn;
+    int threads;
+    size_t smem;
+};
+
+// Which variant writes the rows of a graph of n vertices.  Two vertices a thread
+// where the rows' 16-byte stores are aligned and that still fills the device
+// (scale 24 rows 3.68 -> 3.04 ms); on small graphs smaller blocks, so that more of
+// them share the work.
+MsRows ms_rows(int64_t n)
+{
+    const size_t entry = kMatSlots * sizeof(uint2);
+    if (n < 148 * 256) { return {ms_materialize_kernel<1, 64>, 64, 64 * entry}; }
+    if (n % 2 == 0 && n >= 148 * 3 * 512) { return {ms_materialize_kernel<2, 256>, 256, 512 * entry}; }
+    return {ms_materialize_kernel<1, 256>, 256, 256 * entry};
 }
 
 using MsKernel = void (*)(MsParams);
@@ -1473,7 +1562,8 @@ bd_status ms_enqueue_materialize(bd_msbfs *b, int group, int count)
     o.lanes = count;
     o.depth_out = b->out_depth + (int64_t)group * 64 * n;
     o.parent_out = b->out_parent + (int64_t)group * 64 * n;
-    ms_materialize_kernel<<<b->mat_grid, kMatThreads, kMatSmem, b->stream>>>(o);
+    const MsRows rows = ms_rows(n);
+    rows.fn<<<b->mat_grid, rows.threads, rows.smem, b->stream>>>(o);
     BD_CUDA(cudaGetLastError());
     if (b->opts.min_parent) {
         for (int r = 0; r < count; ++r) {
@@ -1738,10 +1828,11 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
     if (!ok) { return fail(BD_ERR_OOM); }
     if (o.materialize) {
         int per_sm = 0, sms = 0;
-        if (cudaFuncSetAttribute(ms_materialize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kMatSmem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_materialize_kernel,
-                                                          kMatThreads, kMatSmem) != cudaSuccess ||
+        const MsRows rows = ms_rows(n);
+        if (cudaFuncSetAttribute((const void *)rows.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)rows.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)rows.fn, rows.threads,
+                                                          rows.smem) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess ||
             per_sm < 1) {
             return fail(BD_ERR_CUDA);
