@@ -1,7 +1,7 @@
 // bd_bfs.cu -- the B200 direction-optimizing BFS (hybrid_bfs) and its C ABI.
 //
 // Data layout in HBM for one handle (n vertices, arcs = 2m):
-//   depth   int32[n]      -1 = unvisited; claimed by atomicCAS in top-down
+//   depth   int32[n]      -1 = unvisited
 //   parent  int64[n]      written once per reached vertex; the reference's
 //                         -deg / -1 encoding of unreached vertices is filled
 //                         in lazily (finalize_parents_kernel) when read
@@ -164,9 +164,11 @@ struct Team {
 constexpr int kILP = 4;
 
 // Top-down claims of a batch of kILP neighbours per lane (hybrid_bfs.cc:83-96):
-// visited-bit filter, then atomicCAS on the depth word decides the single
-// winner, which writes the parent, sets the visited bit and joins the next
-// frontier.  Every stage issues its kILP memory operations back to back.
+// visited-bit filter, then the atomicOr that sets the bit decides the single
+// winner, which writes depth and parent and joins the next frontier.  Every
+// stage issues its kILP memory operations back to back.  (Claiming by atomicCAS
+// on the depth word and setting the bit afterwards took a second atomic per
+// winner and a scattered sector per loser.)
 __device__ __forceinline__ void td_claim_batch(const BfsParams &p, Acc *acc, uint32_t *vis,
                                                int qout, int new_level, const bool (&ok)[kILP],
                                                const uint32_t (&v)[kILP],
@@ -175,21 +177,21 @@ __device__ __forceinline__ void td_claim_batch(const BfsParams &p, Acc *acc, uin
     uint32_t w[kILP];
 #pragma unroll
     for (int i = 0; i < kILP; ++i) { w[i] = ok[i] ? __ldcg(&vis[v[i] >> 5]) : 0xFFFFFFFFu; }
-    int old[kILP];
+    bool won[kILP];
 #pragma unroll
     for (int i = 0; i < kILP; ++i) {
-        const bool cand = ok[i] && !((w[i] >> (v[i] & 31)) & 1u);
-        old[i] = cand ? atomicCAS(&p.depth[v[i]], -1, new_level) : 0;
+        const uint32_t bit = 1u << (v[i] & 31);
+        won[i] = !(w[i] & bit);  // arcs past the list read as visited
+        if (won[i]) { w[i] = atomicOr(&vis[v[i] >> 5], bit); }
     }
-    bool won[kILP];
     int64_t deg[kILP];
 #pragma unroll
     for (int i = 0; i < kILP; ++i) {
-        won[i] = ok[i] && !((w[i] >> (v[i] & 31)) & 1u) && old[i] == -1;
+        won[i] = won[i] && !((w[i] >> (v[i] & 31)) & 1u);
         deg[i] = 0;
         if (won[i]) {
+            p.depth[v[i]] = new_level;
             p.parent[v[i]] = (int64_t)src[i];
-            atomicOr(&vis[v[i] >> 5], 1u << (v[i] & 31));
             deg[i] = degree_of(p, v[i]);
         }
     }
@@ -1476,23 +1478,65 @@ __global__ void finalize_parents_kernel(const int64_t *off, int64_t n, const int
     }
 }
 
-// BD_ORDER_HUB: depths and parents in the caller's numbering (traversal
-// arrays are indexed, and parents named, by traversal id), with the
-// reference's encoding of unreached vertices.
-__global__ void hub_outputs_kernel(const uint32_t *perm, const uint32_t *iperm, const int64_t *off,
-                                   int64_t n, const int32_t *depth, const int64_t *parent,
-                                   int32_t *out_depth, int64_t *out_parent)
+// Depths and parents in the caller's arrays and numbering, with the reference's
+// encoding of unreached vertices.  HUB (BD_ORDER_HUB): the traversal arrays are
+// indexed, and parents named, by traversal id.  A thread takes V consecutive
+// vertices with each stage's reads issued together (V = 4: 16-byte accesses to the
+// caller's arrays, which have to be aligned for them): bound by the random sectors
+// of depth, parent and numbering, which one vertex a thread left waiting on one
+// chain of four reads.
+template <bool HUB, int V>
+__global__ void __launch_bounds__(256) outputs_kernel(const uint32_t *perm, const uint32_t *iperm,
+                                                      const int64_t *off, int64_t n,
+                                                      const int32_t *depth, const int64_t *parent,
+                                                      int32_t *out_depth, int64_t *out_parent)
 {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t t = perm[v];
-        const int32_t d = depth[t];
-        out_depth[v] = d;
-        if (d >= 0) {
-            out_parent[v] = (int64_t)iperm[parent[t]];
+    static_assert(V == 1 || V == 4, "one vertex or four");
+    for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * V; v < n;
+         v += (int64_t)gridDim.x * blockDim.x * V) {
+        int64_t t[V];
+        if constexpr (HUB && V == 4) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(perm + v));
+            t[0] = q.x;
+            t[1] = q.y;
+            t[2] = q.z;
+            t[3] = q.w;
         } else {
-            const int64_t deg = off[v + 1] - off[v];
-            out_parent[v] = deg != 0 ? -deg : -1;
+#pragma unroll
+            for (int i = 0; i < V; ++i) { t[i] = HUB ? (int64_t)__ldg(&perm[v + i]) : v + i; }
+        }
+        int32_t d[V];
+        int64_t par[V];
+        bool all = true;
+#pragma unroll
+        for (int i = 0; i < V; ++i) { d[i] = __ldg(&depth[t[i]]); }
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            par[i] = d[i] >= 0 ? __ldg(&parent[t[i]]) : 0;
+            all = all && d[i] >= 0;
+        }
+        if constexpr (HUB) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                if (d[i] >= 0) { par[i] = (int64_t)__ldg(&iperm[par[i]]); }
+            }
+        }
+        if (!all) {
+            int64_t o[V + 1];
+#pragma unroll
+            for (int i = 0; i <= V; ++i) { o[i] = __ldg(&off[v + i]); }
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                if (d[i] < 0) { par[i] = o[i + 1] != o[i] ? o[i] - o[i + 1] : -1; }
+            }
+        }
+        if constexpr (V == 4) {
+            *reinterpret_cast<int4 *>(out_depth + v) = make_int4(d[0], d[1], d[2], d[3]);
+            *reinterpret_cast<longlong2 *>(out_parent + v) = make_longlong2(par[0], par[1]);
+            *reinterpret_cast<longlong2 *>(out_parent + v + 2) = make_longlong2(par[2], par[3]);
+        } else {
+            out_depth[v] = d[0];
+            out_parent[v] = par[0];
         }
     }
 }
@@ -1514,6 +1558,20 @@ int grid_for(int64_t items, int threads = 256)
     if (b < 1) { b = 1; }
     if (b > 148 * 32) { b = 148 * 32; }
     return (int)b;
+}
+
+// outputs_kernel for a graph's layout and the caller's arrays.
+cudaError_t launch_outputs(const bd_graph *g, const int32_t *depth, const int64_t *parent,
+                           int32_t *out_depth, int64_t *out_parent, cudaStream_t s)
+{
+    const int64_t n = g->n;
+    const bool wide = n % 4 == 0 && (reinterpret_cast<uintptr_t>(out_depth) |
+                                     reinterpret_cast<uintptr_t>(out_parent)) % 16 == 0;
+    auto fn = g->d_perm ? (wide ? outputs_kernel<true, 4> : outputs_kernel<true, 1>)
+                        : (wide ? outputs_kernel<false, 4> : outputs_kernel<false, 1>);
+    fn<<<grid_for(wide ? n / 4 : n), 256, 0, s>>>(g->d_perm, g->d_iperm, g->d_off, n, depth, parent,
+                                                  out_depth, out_parent);
+    return cudaGetLastError();
 }
 
 using KernelFn = void (*)(BfsParams);
@@ -1663,24 +1721,6 @@ bd_status ensure_sources(bd_bfs *b, int64_t count)
     return BD_OK;
 }
 
-// Depths and parents in the caller's arrays with the reference's encoding
-// of unreached vertices (graphs without a hub numbering: the same ids).
-__global__ void copy_outputs_kernel(const int64_t *off, int64_t n, const int32_t *depth,
-                                    const int64_t *parent, int32_t *out_depth, int64_t *out_parent)
-{
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t d = depth[v];
-        out_depth[v] = d;
-        if (d >= 0) {
-            out_parent[v] = parent[v];
-        } else {
-            const int64_t deg = off[v + 1] - off[v];
-            out_parent[v] = deg != 0 ? -deg : -1;
-        }
-    }
-}
-
 // Enqueues the persistent kernel (+ min-parent pass) for `count` sources in
 // d_sources, or for the one source given (count 1).  m_c and n_c go to result
 // (device) if given.  With out_depth / out_parent (device, n entries each) the results are also written there
@@ -1705,30 +1745,17 @@ bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t star
     BD_CUDA(cudaLaunchCooperativeKernel((const void *)b->kernel.fn, dim3(b->grid),
                                         dim3(b->kernel.block), args, b->kernel.smem, b->stream));
     if (out_depth) {
-        const int64_t n = b->g->n;
-        if (b->g->d_perm) {
-            hub_outputs_kernel<<<grid_for(n), 256, 0, b->stream>>>(
-                b->g->d_perm, b->g->d_iperm, b->g->d_off, n, b->depth, b->parent, out_depth,
-                out_parent);
-        } else {
-            copy_outputs_kernel<<<grid_for(n), 256, 0, b->stream>>>(b->g->d_off, n, b->depth,
-                                                                   b->parent, out_depth, out_parent);
-        }
-        BD_CUDA(cudaGetLastError());
+        BD_CUDA(launch_outputs(b->g, b->depth, b->parent, out_depth, out_parent, b->stream));
         if (b->opts.min_parent) {
             BD_CUDA(launch_min_parent(b->g, b->min_scratch, out_depth, out_parent, b->stream));
         }
     } else if (b->opts.min_parent) {
         // the smallest parent in the caller's numbering: on a hub graph, map
         // the outputs back first, then pick parents on the caller's CSR
-        const int64_t n = b->g->n;
         int32_t *depth = b->depth;
         int64_t *parent = b->parent;
         if (b->out_depth) {
-            hub_outputs_kernel<<<grid_for(n), 256, 0, b->stream>>>(
-                b->g->d_perm, b->g->d_iperm, b->g->d_off, n, b->depth, b->parent, b->out_depth,
-                b->out_parent);
-            BD_CUDA(cudaGetLastError());
+            BD_CUDA(launch_outputs(b->g, depth, parent, b->out_depth, b->out_parent, b->stream));
             depth = b->out_depth;
             parent = b->out_parent;
         }
@@ -1791,9 +1818,7 @@ bd_status finalize_parents(bd_bfs *b)
     if (b->parents_final) { return BD_OK; }
     const int64_t n = b->g->n;
     if (b->out_depth) {
-        hub_outputs_kernel<<<grid_for(n), 256, 0, b->stream>>>(
-            b->g->d_perm, b->g->d_iperm, b->g->d_off, n, b->depth, b->parent, b->out_depth,
-            b->out_parent);
+        BD_CUDA(launch_outputs(b->g, b->depth, b->parent, b->out_depth, b->out_parent, b->stream));
     } else {
         finalize_parents_kernel<<<grid_for(n), 256, 0, b->stream>>>(b->g->d_off, n, b->depth,
                                                                   b->parent);
