@@ -1262,7 +1262,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) bfs_persistent_kernel(
     }
     __syncthreads();
     if (sh.consult) { return; }
-    const Team grid{(long long)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5),
+    // consecutive ranks on different CTAs: a narrow level's few work items then
+    // spread over the SMs instead of filling some
+    const Team grid{(long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x,
                     (long long)gridDim.x * (BLOCK / 32), nullptr};
     bool init = true;
     Local loc{0, 0};

@@ -305,6 +305,16 @@ __device__ __forceinline__ MsView ms_view(const MsState &c)
     return v;
 }
 
+// This warp among the grid's, consecutive ranks on different CTAs: work items are
+// few on narrow levels, and their heavy ones stand together (the first words of a
+// hub numbering), so ranks that fill one CTA after another put them on a few SMs,
+// whose request rate then bounds the level (the first pull of 64 roots at scale 16:
+// 30 us in CTA 0, under 5 in most others).
+__device__ __forceinline__ long long ms_warp_rank()
+{
+    return (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+}
+
 // Zeroes the frontier words of the frontier read by the previous step.
 __device__ void ms_clear_old(const MsParams &p, const MsView &sv)
 {
@@ -418,8 +428,7 @@ template <int BLOCK>
 __device__ void ms_push_step(const MsParams &p, const MsView &sv, MsWarpScratch &ws, MsLocal &loc)
 {
     const int lane = lane_id();
-    const int warp = threadIdx.x >> 5;
-    const long long gw = (long long)blockIdx.x * (BLOCK / 32) + warp;
+    const long long gw = ms_warp_rank();
     const long long nw = (long long)gridDim.x * (BLOCK / 32);
     const int cur = sv.step % 3, nxt = (sv.step + 1) % 3;
     MsAcc *acc = &p.ctrl->acc[sv.step % 3];
@@ -496,8 +505,7 @@ template <int BLOCK>
 __device__ void ms_pull_long(const MsParams &p, const MsView &sv, MsLocal &loc)
 {
     const int lane = lane_id();
-    const int warp = threadIdx.x >> 5;
-    const long long gw = (long long)blockIdx.x * (BLOCK / 32) + warp;
+    const long long gw = ms_warp_rank();
     const long long nw = (long long)gridDim.x * (BLOCK / 32);
     const int cur = sv.step % 3, nxt = (sv.step + 1) % 3;
     MsAcc *acc = &p.ctrl->acc[sv.step % 3];
@@ -620,7 +628,7 @@ __device__ void ms_pull_step(const MsParams &p, const MsView &sv, MsLocal &loc)
     // chunk per warp would leave most warps idle).  Either way a warp loads
     // 32 skip masks at once (one per lane) and walks only the words with
     // work: done vertices have nothing to do.
-    const long long gw = (long long)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5);
+    const long long gw = ms_warp_rank();
     const long long nw = (long long)gridDim.x * (BLOCK / 32);
     const long long chunks = (words + 31) / 32;
     const bool dynamic = chunks >= 2 * nw;
