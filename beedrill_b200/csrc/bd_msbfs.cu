@@ -1856,25 +1856,29 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
     }
     b->grid = per_sm * sms;
     // Where a pull scan leaves a list to all warps (0 = this rule).  A warp takes
-    // a word of 32 vertices, so up to 32 x heavy_degree arcs one after another;
-    // that should not exceed what the average warp scans in a full pull, arcs /
-    // warps.  64 roots on the hub layout, traversal ms by heavy_degree:
-    //   scale 16 (rule 32)    32: 0.18   64: 0.20   256: 0.28   4096: 0.73
-    //   scale 20 (rule 218)   96: 0.48   192: 0.46  512: 0.53   4096: 1.37
-    //   scale 22 (rule 886)  256: 1.14   512: 1.13  1024: 1.19  4096: 1.40
-    //   scale 24 (rule 3430) 512: 3.66  1024: 3.61  4096: 3.56
-    // (scales 20 and 22: batches with a lane whose frontier is still small).
-    // Shorter lists than 32 arcs are not worth a chunk; above 4096 arcs even the
-    // largest graphs gain by dealing them out.
-    const int64_t warps = (int64_t)b->grid * (b->block / 32);
+    // a word of 32 vertices, so up to 32 x heavy_degree arcs one after another,
+    // to be held against the arcs an average warp scans in a full pull (arcs /
+    // warps): a word may take a good third of that where the scans are bound by
+    // latency, the whole of it on graphs far beyond L2, where leaving a list
+    // early costs re-reads.  Traversal ms by heavy_degree, hub layout, 64 roots
+    // (scale 16) and sums over four batches:
+    //   scale 16 (rule 32)    32: 0.14   64: 0.15   256: 0.28   4096: 0.73
+    //   scale 20 (rule 83)    64: 1.74  256: 1.83   512: 1.92   1024: 2.19
+    //   scale 22 (rule 354)  128: 4.83  256: 4.81   512: 4.82   1024: 4.97
+    //   scale 24 (rule 3430) 512: 16.98 1024: 16.87 4096: 16.69
+    // Lists up to 1024 arcs in a numbering that does not put the hubs together are
+    // not left at all: a word then holds one or two of them, which take less time
+    // than the barrier (scale 12, degree order: 0.111 against 0.097 ms).
+    const int64_t per_warp = g->arcs / ((int64_t)b->grid * (b->block / 32));
     if (b->opts.heavy_degree <= 0) {
-        b->opts.heavy_degree =
-            (int32_t)std::min<int64_t>(4096, std::max<int64_t>(32, g->arcs / (32 * warps)));
+        b->opts.heavy_degree = (int32_t)std::min<int64_t>(
+            4096, std::max<int64_t>(32, per_warp < 65536 ? per_warp / 80 : per_warp / 32));
+        if (!g->d_perm && g->max_degree <= 1024) { b->opts.heavy_degree = 1024; }
     }
-    // chunks of a few such lengths: scale 16 128 arcs 0.18, 512 0.20; scale 20
-    // 128: 0.40, 512: 0.39
+    // chunks of about two such lengths (scale 22, heavy_degree 512: 4.59 with 512
+    // arcs, 4.63 with 2048)
     if (b->opts.heavy_chunk <= 0) {
-        b->opts.heavy_chunk = std::min(2048, std::max(128, 4 * b->opts.heavy_degree));
+        b->opts.heavy_chunk = std::min(2048, std::max(128, 2 * b->opts.heavy_degree));
     }
     b->opts.pull_prefix = std::min(b->opts.pull_prefix, b->opts.heavy_degree);
     // room for every chunk a pull step can leave to ms_pull_long
