@@ -191,6 +191,7 @@ def lib() -> ctypes.CDLL:
         "bd_msbfs_get_depths": (c_int, [c_void_p, c_int32, i32p]),
         "bd_msbfs_get_parents": (c_int, [c_void_p, c_int32, i64p]),
         "bd_msbfs_count_traversed_edges": (c_int, [c_void_p, c_int32, i64p, i64p]),
+        "bd_msbfs_counts": (c_int, [c_void_p, i64p, i64p]),
         "bd_msbfs_get_steps": (c_int, [c_void_p, POINTER(Step), c_int64, i64p]),
         "bd_msbfs_check": (c_int, [c_void_p, c_int32, POINTER(c_int32)]),
         "bd_msbfs_device_results": (c_int, [c_void_p, c_int32, vpp, vpp]),
@@ -640,10 +641,7 @@ class BatchedBFS:
         """(m_c, n_c) arrays over the roots of the last run."""
         m = np.empty(self.count, np.int64)
         n = np.empty(self.count, np.int64)
-        for i in range(self.count):
-            e, r = c_int64(), c_int64()
-            _check(lib().bd_msbfs_count_traversed_edges(self._h, i, byref(e), byref(r)), "count")
-            m[i], n[i] = e.value, r.value
+        _check(lib().bd_msbfs_counts(self._h, _ptr(m, c_int64), _ptr(n, c_int64)), "count")
         return m, n
 
     def steps(self) -> list[dict]:

@@ -1637,6 +1637,11 @@ struct bd_bfs {
     bd_step *rec = nullptr;
     int64_t *d_sources = nullptr;
     int64_t sources_cap = 0;
+    // run_many: a pair of events and of results per root, kept for the next call
+    std::vector<cudaEvent_t> events;
+    int64_t *d_results = nullptr;
+    int64_t results_cap = 0;
+    CtrlHead *head = nullptr;  // pinned: where a run's outcome is read back to
     PolicyBlob *policy = nullptr;  // device copy, or null
     KernelChoice kernel{nullptr, 0, 0};
     int grid = 0;
@@ -1652,7 +1657,7 @@ struct bd_bfs {
     bool ran = false;
     bool parents_final = false;  // caller-visible depths and parents are up to date
     int64_t last_source = -1;
-    Ctrl last{};
+    CtrlHead last{};
 };
 
 namespace bd {
@@ -1770,10 +1775,17 @@ bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t star
     return BD_OK;
 }
 
+// Queues the read-back of a run's outcome behind it; the caller waits for the
+// stream once, for this and whatever else it queued.
+bd_status enqueue_collect(bd_bfs *b)
+{
+    BD_CUDA(cudaMemcpyAsync(b->head, b->ctrl, sizeof(CtrlHead), cudaMemcpyDeviceToHost, b->stream));
+    return BD_OK;
+}
+
 bd_status collect(bd_bfs *b, bd_run_stats *stats, double ms)
 {
-    BD_CUDA(cudaMemcpyAsync(&b->last, b->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, b->stream));
-    BD_CUDA(cudaStreamSynchronize(b->stream));
+    b->last = *b->head;
     b->ran = true;
     b->cleared = false;
     // a min-parent run on a hub graph wrote the caller-order outputs itself
@@ -1807,15 +1819,16 @@ bd_status run_sources(bd_bfs *b, const int64_t *sources, int64_t count, bd_run_s
                                 cudaMemcpyHostToDevice, b->stream));
     }
     BD_TRY(enqueue_bfs(b, count, sources[0], b->ev0, b->ev1));
-    BD_CUDA(cudaEventSynchronize(b->ev1));
+    BD_TRY(enqueue_collect(b));
+    BD_CUDA(cudaStreamSynchronize(b->stream));
     float ms = 0.f;
     BD_CUDA(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
     b->last_source = count == 1 ? sources[0] : -1;
     return collect(b, stats, (double)ms);
 }
 
-// Makes the caller-visible depths and parents current: the reference's
-// -deg / -1 encoding of unreached vertices, and on a hub graph the mapping
+// Makes the caller-visible depths and parents current (queued on the handle's
+// stream): the reference's -deg / -1 encoding of unreached vertices, and on a hub graph the mapping
 // back to the caller's numbering.
 bd_status finalize_parents(bd_bfs *b)
 {
@@ -1829,8 +1842,7 @@ bd_status finalize_parents(bd_bfs *b)
                                                                   b->parent);
     }
     BD_CUDA(cudaGetLastError());
-    BD_CUDA(cudaStreamSynchronize(b->stream));
-    b->parents_final = true;
+    b->parents_final = true;  // in stream order
     return BD_OK;
 }
 
@@ -1852,6 +1864,9 @@ void bfs_free(bd_bfs *b)
     cudaFree(b->ctrl);
     cudaFree(b->rec);
     cudaFree(b->d_sources);
+    cudaFree(b->d_results);
+    for (cudaEvent_t e : b->events) { cudaEventDestroy(e); }
+    if (b->head) { cudaFreeHost(b->head); }
     cudaFree(b->policy);
     min_parent_free(&b->min_scratch);
     check_free(&b->check);
@@ -1942,6 +1957,7 @@ bd_status bd_bfs_create(bd_graph *g, const bd_bfs_opts *opts, bd_bfs **out)
               (!g->d_perm || (cudaMalloc(&b->out_depth, sizeof(int32_t) * n) == cudaSuccess &&
                               cudaMalloc(&b->out_parent, sizeof(int64_t) * n) == cudaSuccess)) &&
               cudaMalloc(&b->ctrl, sizeof(Ctrl)) == cudaSuccess &&
+              cudaHostAlloc(&b->head, sizeof(CtrlHead), cudaHostAllocDefault) == cudaSuccess &&
               cudaMalloc(&b->rec, sizeof(bd_step) * kRecCap) == cudaSuccess &&
               (!o.min_parent || min_parent_alloc(g, &b->min_scratch) == cudaSuccess);
     for (int i = 0; i < 2 && ok; ++i) {
@@ -2017,6 +2033,25 @@ bd_status bd_bfs_run_bottom_up(bd_bfs *b, int64_t source, bd_run_stats *stats)
 namespace bd {
 namespace {
 
+constexpr int64_t kKeptEvents = 2050;  // a handle keeps events for 1024 roots
+
+// Events and result slots for k roots.
+bd_status ensure_many(bd_bfs *b, int64_t k)
+{
+    while ((int64_t)b->events.size() < 2 * k + 2) {
+        cudaEvent_t e = nullptr;
+        BD_CUDA(cudaEventCreate(&e));
+        b->events.push_back(e);
+    }
+    if (k <= b->results_cap) { return BD_OK; }
+    cudaFree(b->d_results);
+    b->d_results = nullptr;
+    b->results_cap = 0;
+    BD_CUDA(cudaMalloc(&b->d_results, sizeof(int64_t) * 2 * k));
+    b->results_cap = k;
+    return BD_OK;
+}
+
 bd_status run_many(bd_bfs *b, const int64_t *sources, int64_t k, int32_t *d_depth,
                    int64_t *d_parent, double *ms_out, int64_t *edges_out, int64_t *reached_out,
                    double *e2e_ms)
@@ -2026,26 +2061,12 @@ bd_status run_many(bd_bfs *b, const int64_t *sources, int64_t k, int32_t *d_dept
         if (sources[i] < 0 || sources[i] >= b->g->n) { return BD_ERR_RANGE; }
     }
     BD_CUDA(cudaSetDevice(b->device));
-    int64_t *d_edges = nullptr;
-    std::vector<cudaEvent_t> ev(2 * k, nullptr);
-    bd_status st = BD_OK;
-    cudaEvent_t wall0 = nullptr, wall1 = nullptr;
-    auto cleanup = [&]() {
-        for (auto e : ev) { if (e) { cudaEventDestroy(e); } }
-        if (wall0) { cudaEventDestroy(wall0); }
-        if (wall1) { cudaEventDestroy(wall1); }
-        cudaFree(d_edges);
-    };
-    if (cudaMalloc(&d_edges, sizeof(int64_t) * 2 * k) != cudaSuccess ||
-        cudaEventCreate(&wall0) != cudaSuccess || cudaEventCreate(&wall1) != cudaSuccess) {
-        cleanup();
-        return BD_ERR_OOM;
-    }
-    for (auto &e : ev) {
-        if (cudaEventCreate(&e) != cudaSuccess) { cleanup(); return BD_ERR_CUDA; }
-    }
+    bd_status st = ensure_many(b, k);
+    if (st != BD_OK) { return st; }
+    const std::vector<cudaEvent_t> &ev = b->events;  // 2 per root, then the call's 2
+    int64_t *d_edges = b->d_results;
     std::vector<int64_t> host_edges(2 * k);
-    cudaEventRecord(wall0, b->stream);
+    cudaEventRecord(ev[2 * k], b->stream);
     const int64_t n = b->g->n;
     for (int64_t i = 0; i < k && st == BD_OK; ++i) {
         st = enqueue_clear(b);
@@ -2058,13 +2079,13 @@ bd_status run_many(bd_bfs *b, const int64_t *sources, int64_t k, int32_t *d_dept
     if (st == BD_OK &&
         (cudaMemcpyAsync(host_edges.data(), d_edges, sizeof(int64_t) * 2 * k, cudaMemcpyDeviceToHost,
                          b->stream) != cudaSuccess ||
-         cudaEventRecord(wall1, b->stream) != cudaSuccess ||
-         cudaStreamSynchronize(b->stream) != cudaSuccess)) {
+         cudaEventRecord(ev[2 * k + 1], b->stream) != cudaSuccess ||
+         enqueue_collect(b) != BD_OK || cudaStreamSynchronize(b->stream) != cudaSuccess)) {
         st = BD_ERR_CUDA;
     }
     if (st == BD_OK) {
         float w = 0.f;
-        cudaEventElapsedTime(&w, wall0, wall1);
+        cudaEventElapsedTime(&w, ev[2 * k], ev[2 * k + 1]);
         if (e2e_ms) { *e2e_ms = (double)w; }
         for (int64_t i = 0; i < k; ++i) {
             float ms = 0.f;
@@ -2076,7 +2097,10 @@ bd_status run_many(bd_bfs *b, const int64_t *sources, int64_t k, int32_t *d_dept
         b->last_source = sources[k - 1];
         st = collect(b, nullptr, 0.0);
     }
-    cleanup();
+    while ((int64_t)b->events.size() > kKeptEvents) {
+        cudaEventDestroy(b->events.back());
+        b->events.pop_back();
+    }
     return st;
 }
 
@@ -2105,8 +2129,9 @@ bd_status bd_bfs_get_depths(bd_bfs *b, int32_t *depth)
     if (!b->ran) { return BD_ERR_STATE; }
     BD_CUDA(cudaSetDevice(b->device));
     BD_TRY(finalize_parents(b));
-    BD_CUDA(cudaMemcpy(depth, b->out_depth ? b->out_depth : b->depth, sizeof(int32_t) * b->g->n,
-                       cudaMemcpyDeviceToHost));
+    BD_CUDA(cudaMemcpyAsync(depth, b->out_depth ? b->out_depth : b->depth,
+                            sizeof(int32_t) * b->g->n, cudaMemcpyDeviceToHost, b->stream));
+    BD_CUDA(cudaStreamSynchronize(b->stream));
     return BD_OK;
 }
 
@@ -2115,8 +2140,9 @@ bd_status bd_bfs_get_parents(bd_bfs *b, int64_t *parent)
     if (!b || !parent) { return BD_ERR_INVALID; }
     BD_CUDA(cudaSetDevice(b->device));
     BD_TRY(finalize_parents(b));
-    BD_CUDA(cudaMemcpy(parent, b->out_parent ? b->out_parent : b->parent,
-                       sizeof(int64_t) * b->g->n, cudaMemcpyDeviceToHost));
+    BD_CUDA(cudaMemcpyAsync(parent, b->out_parent ? b->out_parent : b->parent,
+                            sizeof(int64_t) * b->g->n, cudaMemcpyDeviceToHost, b->stream));
+    BD_CUDA(cudaStreamSynchronize(b->stream));
     return BD_OK;
 }
 
@@ -2125,6 +2151,7 @@ bd_status bd_bfs_device_ptrs(bd_bfs *b, const int32_t **depth, const int64_t **p
     if (!b) { return BD_ERR_INVALID; }
     BD_CUDA(cudaSetDevice(b->device));
     BD_TRY(finalize_parents(b));
+    BD_CUDA(cudaStreamSynchronize(b->stream));
     if (depth) { *depth = b->out_depth ? b->out_depth : b->depth; }
     if (parent) { *parent = b->out_parent ? b->out_parent : b->parent; }
     return BD_OK;
@@ -2331,8 +2358,8 @@ extern "C" bd_status bd_bfs_run_noalloc(const int64_t *d_offsets, const uint32_t
     finalize_parents_kernel<<<grid_for(num_vertices), 256, 0, s>>>(d_offsets, num_vertices, d_depth,
                                                                    d_parent);
     BD_CUDA(cudaGetLastError());
-    Ctrl host{};
-    BD_CUDA(cudaMemcpyAsync(&host, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
+    CtrlHead host{};
+    BD_CUDA(cudaMemcpyAsync(&host, ctrl, sizeof(CtrlHead), cudaMemcpyDeviceToHost, s));
     BD_CUDA(cudaStreamSynchronize(s));
     if (host.error) { return (bd_status)host.error; }
     if (traversed_edges) { *traversed_edges = host.st.visited_degsum / 2; }

@@ -71,13 +71,16 @@ struct LevelState {
     long long barrier;           // number of the next grid barrier
 };
 
-// Device-resident control block of one BFS handle.
-struct alignas(16) Ctrl {
+// Device-resident control block of one BFS handle; its head is what the host
+// reads after a run.
+struct alignas(16) CtrlHead {
     unsigned long long bar;      // arrivals; barrier b is complete at (b + 1) * CTAs
     int error;
     int pad0;
     long long barrier;           // number of the next launch's first barrier
-    LevelState st;               // the final state, for the host
+    LevelState st;               // the final state
+};
+struct Ctrl : CtrlHead {
     LevelState pub[2];           // published by CTA 0 at barrier b, in slot b % 2
     Acc acc[3];
 };

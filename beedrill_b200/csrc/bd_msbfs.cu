@@ -87,12 +87,23 @@ struct MsState {
     long long bars;              // grid barriers passed
 };
 
-struct MsCtrl {
+// The control block; its head is what the host reads after a run.
+struct alignas(16) MsCtrlHead {
     ull bar;       // barrier arrivals; barrier b is complete at (b + 1) * CTAs
     int error, pad0;
     ull t_start;   // min over CTAs of their start time
     MsState st;
+};
+struct MsCtrl : MsCtrlHead {
     MsAcc acc[3];
+};
+
+// Pinned host memory of a call: the group's sources (64 each), the per-lane counts
+// (128 each) and the head of the control block.
+struct MsHostIo {
+    MsCtrlHead head;
+    int64_t *sources;
+    ull *counts;
 };
 
 struct MsParams {
@@ -1488,7 +1499,8 @@ struct bd_msbfs {
     int graph_count = -1;
     bool graph_ok = true;
     bool frontier_clean = false;  // F is all zero (kernels leave it so)
-    MsCtrl last{};
+    MsCtrlHead last{};
+    MsHostIo *io = nullptr;  // pinned, with its arrays behind it
     std::vector<unsigned long long> counts;
     // opts.materialize: every root's results, written by each run
     int32_t *out_depth = nullptr;   // [max_roots][n]
@@ -1680,6 +1692,7 @@ void ms_free(bd_msbfs *b)
     cudaFree(b->rec);
     cudaFree(b->d_sources);
     cudaFree(b->d_counts);
+    if (b->io) { cudaFreeHost(b->io); }
     cudaFree(b->policy);
     cudaFree(b->dq);
     min_parent_free(&b->min_scratch);
@@ -1833,6 +1846,16 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
     } else if (ok) {
         ok = cudaMalloc(&b->xbuf, sizeof(int64_t) * n) == cudaSuccess;
     }
+    if (ok) {
+        void *io = nullptr;
+        ok = cudaHostAlloc(&io, sizeof(MsHostIo) + (size_t)b->groups * (64 * sizeof(int64_t) + 128 * sizeof(ull)),
+                           cudaHostAllocDefault) == cudaSuccess;
+        if (ok) {
+            b->io = static_cast<MsHostIo *>(io);
+            b->io->sources = reinterpret_cast<int64_t *>(b->io + 1);
+            b->io->counts = reinterpret_cast<ull *>(b->io->sources + 64 * b->groups);
+        }
+    }
     if (!ok) { return fail(BD_ERR_OOM); }
     if (o.materialize) {
         int per_sm = 0, sms = 0;
@@ -1902,19 +1925,20 @@ bd_status bd_msbfs_run(bd_msbfs *b, const int64_t *sources, int32_t count, bd_ru
     }
     BD_CUDA(cudaSetDevice(b->device));
     // group g's sources start at d_sources + 64 g
-    std::vector<int64_t> padded((size_t)64 * b->groups, 0);
-    for (int i = 0; i < count; ++i) { padded[(size_t)(i / 64) * 64 + i % 64] = sources[i]; }
-    BD_CUDA(cudaMemcpyAsync(b->d_sources, padded.data(), sizeof(int64_t) * padded.size(),
+    std::copy(sources, sources + count, b->io->sources);
+    BD_CUDA(cudaMemcpyAsync(b->d_sources, b->io->sources, sizeof(int64_t) * count,
                             cudaMemcpyHostToDevice, b->stream));
     BD_CUDA(cudaEventRecord(b->ev0, b->stream));
     BD_TRY(ms_launch(b, count));
     BD_CUDA(cudaEventRecord(b->ev1, b->stream));
     const int used = (count + 63) / 64;
-    b->counts.assign((size_t)128 * used, 0);
-    BD_CUDA(cudaMemcpyAsync(b->counts.data(), b->d_counts, sizeof(unsigned long long) * 128 * used,
+    BD_CUDA(cudaMemcpyAsync(b->io->counts, b->d_counts, sizeof(ull) * 128 * used,
                             cudaMemcpyDeviceToHost, b->stream));
-    BD_CUDA(cudaMemcpyAsync(&b->last, b->ctrl, sizeof(MsCtrl), cudaMemcpyDeviceToHost, b->stream));
+    BD_CUDA(cudaMemcpyAsync(&b->io->head, b->ctrl, sizeof(MsCtrlHead), cudaMemcpyDeviceToHost,
+                            b->stream));
     BD_CUDA(cudaStreamSynchronize(b->stream));
+    b->counts.assign(b->io->counts, b->io->counts + 128 * used);
+    b->last = b->io->head;
     b->count = count;
     b->sources.assign(sources, sources + count);
     b->ran = true;
@@ -1985,6 +2009,17 @@ bd_status bd_msbfs_count_traversed_edges(bd_msbfs *b, int32_t root_index, int64_
     const size_t base = (size_t)(root_index / 64) * 128;
     if (edges) { *edges = (int64_t)(b->counts[base + 64 + root_index % 64] / 2); }
     if (reached) { *reached = (int64_t)b->counts[base + root_index % 64]; }
+    return BD_OK;
+}
+
+bd_status bd_msbfs_counts(bd_msbfs *b, int64_t *edges, int64_t *reached)
+{
+    if (!b) { return BD_ERR_INVALID; }
+    if (!b->ran) { return BD_ERR_STATE; }
+    for (int32_t i = 0; i < b->count; ++i) {
+        BD_TRY(bd_msbfs_count_traversed_edges(b, i, edges ? edges + i : nullptr,
+                                              reached ? reached + i : nullptr));
+    }
     return BD_OK;
 }
 
