@@ -285,10 +285,13 @@ __device__ void td_step(const BfsParams &p, const StepView &sv, const Team &team
     const long long nl = sv.f_large;
     const long long nch = sv.f_chunks;
     if (nch > 0) {
-        const long long per = (nch + nw - 1) / nw;
-        const long long c0 = gw * per;
-        const long long c1 = min(nch, c0 + per);
-        if (c0 < c1) {
+        // (x counts parts of chunks where there are too few chunks for the warps)
+        const int cut = split_chunks(nch, p.chunk, nw);
+        const int64_t part = ((int64_t)(p.chunk >> cut) + 31) / 32 * 32;
+        const long long per = ((nch << cut) + nw - 1) / nw;
+        const long long x0 = gw * per, x1 = min(nch << cut, x0 + per);
+        const long long c0 = x0 >> cut;
+        if (x0 < x1) {
             long long lo = 0, hi = nl - 1;  // last i with qlb[i] <= c0
             while (lo < hi) {
                 long long mid = (lo + hi + 1) >> 1;
@@ -297,7 +300,8 @@ __device__ void td_step(const BfsParams &p, const StepView &sv, const Team &team
             long long i = lo;
             long long ibase = (long long)__ldcg(&p.qlb[qin][i]);
             long long inext = i + 1 < nl ? (long long)__ldcg(&p.qlb[qin][i + 1]) : nch;
-            for (long long c = c0; c < c1; ++c) {
+            for (long long x = x0; x < x1; ++x) {
+                const long long c = x >> cut;
                 while (c >= inext) {
                     ++i;
                     ibase = inext;
@@ -305,22 +309,24 @@ __device__ void td_step(const BfsParams &p, const StepView &sv, const Team &team
                 }
                 const uint32_t u = __ldcg(&p.ql[qin][i]);
                 const int64_t ub = __ldg(&p.off[u]), ue = __ldg(&p.off[u + 1]);
-                const int64_t b = ub + (c - ibase) * (int64_t)p.chunk;
-                const int64_t e = min(ue, b + (int64_t)p.chunk);
+                const int64_t cb = ub + (c - ibase) * (int64_t)p.chunk;
+                const int64_t b = cb + (x & ((1ll << cut) - 1)) * part;
+                const int64_t e = min(min(ue, cb + (int64_t)p.chunk), b + part);
                 td_edges_warp(p, acc, vis, qout, new_level, u, b, e, loc);
             }
         }
     }
 
-    // Phase B: small-degree frontier vertices, 32 per warp; their arcs are
+    // Phase B: small-degree frontier vertices, up to 32 per warp; their arcs are
     // laid end to end and dealt to the lanes 32 at a time.
     WarpScratch &ws = sh.warp[warp];
-    for (long long g = gw; g * 32 < sv.f_small; g += nw) {
-        const long long idx = g * 32 + lane;
+    const int group = split_group(sv.f_small, average(sh.st.f_degsum, sh.st.f_count), nw);
+    for (long long g = gw; g << group < sv.f_small; g += nw) {
+        const long long idx = (g << group) + lane;
         uint32_t u = 0;
         int64_t beg = 0;
         int32_t deg = 0;
-        if (idx < sv.f_small) {
+        if (lane >> group == 0 && idx < sv.f_small) {
             u = __ldcg(&p.qs[qin][idx]);
             beg = __ldg(&p.off[u]);
             deg = (int32_t)(__ldg(&p.off[u + 1]) - beg);

@@ -298,6 +298,7 @@ __device__ __forceinline__ void record_shared(const MsParams &p, uint32_t v, ull
 struct MsView {
     int dir, level, step;
     long long f_small, f_large, f_chunks, p_small, p_large;
+    int f_avg;
     ull active;
 };
 
@@ -312,6 +313,7 @@ __device__ __forceinline__ MsView ms_view(const MsState &c)
     v.f_chunks = c.f_chunks;
     v.p_small = c.p_small;
     v.p_large = c.p_large;
+    v.f_avg = dev::average(c.f_degsum, c.f_count);
     v.active = c.active;
     return v;
 }
@@ -444,8 +446,11 @@ __device__ void ms_push_step(const MsParams &p, const MsView &sv, MsWarpScratch 
     const int cur = sv.step % 3, nxt = (sv.step + 1) % 3;
     MsAcc *acc = &p.ctrl->acc[sv.step % 3];
     const int new_level = sv.level + 1;
-    // large frontier vertices: chunk c of vertex ql[i]
-    for (long long c = gw; c < sv.f_chunks; c += nw) {
+    // large frontier vertices: part of chunk c of vertex ql[i]
+    const int cut = split_chunks(sv.f_chunks, p.chunk, nw);
+    const int64_t part = ((int64_t)(p.chunk >> cut) + 31) / 32 * 32;
+    for (long long x = gw; x < sv.f_chunks << cut; x += nw) {
+        const long long c = x >> cut;
         long long lo = 0, hi = sv.f_large - 1;
         while (lo < hi) {
             long long mid = (lo + hi + 1) >> 1;
@@ -454,19 +459,21 @@ __device__ void ms_push_step(const MsParams &p, const MsView &sv, MsWarpScratch 
         const uint32_t u = __ldcg(&p.ql[cur][lo]);
         const long long j = c - (long long)__ldcg(&p.qlb[cur][lo]);
         const ull bits = __ldcg(&p.F[cur][u]);
-        const int64_t ub = __ldg(&p.off[u]), ue = __ldg(&p.off[u + 1]);
-        const int64_t b = ub + j * (int64_t)p.chunk;
-        push_edges(p, acc, cur, nxt, new_level, u, bits, b, min(ue, b + (int64_t)p.chunk), loc);
+        const int64_t ub = __ldg(&p.off[u]) + j * (int64_t)p.chunk;
+        const int64_t ue = min(__ldg(&p.off[u + 1]), ub + (int64_t)p.chunk);
+        const int64_t b = ub + (x & ((1ll << cut) - 1)) * part;
+        push_edges(p, acc, cur, nxt, new_level, u, bits, b, min(ue, b + part), loc);
     }
-    // small frontier vertices, 32 per warp: their lists are laid end to end
+    // small frontier vertices, up to 32 per warp: their lists are laid end to end
     // and dealt to the lanes kPushU x 32 arcs at a time
-    for (long long g = gw; g * 32 < sv.f_small; g += nw) {
-        const long long idx = g * 32 + lane;
+    const int group = split_group(sv.f_small, sv.f_avg, nw);
+    for (long long g = gw; g << group < sv.f_small; g += nw) {
+        const long long idx = (g << group) + lane;
         uint32_t u = 0;
         ull bits = 0;
         int64_t beg = 0;
         int32_t deg = 0;
-        if (idx < sv.f_small) {
+        if (lane >> group == 0 && idx < sv.f_small) {
             u = __ldcg(&p.qs[cur][idx]);
             bits = __ldcg(&p.F[cur][u]);
             beg = __ldg(&p.off[u]);
