@@ -1662,6 +1662,7 @@ struct bd_bfs {
     bool cleared = false;
     bool ran = false;
     bool parents_final = false;  // caller-visible depths and parents are up to date
+    bool rows_by_run = false;    // the last run queued wrote out_depth and out_parent itself
     int64_t last_source = -1;
     CtrlHead last{};
 };
@@ -1777,6 +1778,7 @@ bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t star
         }
         BD_CUDA(launch_min_parent(b->g, b->min_scratch, depth, parent, b->stream));
     }
+    b->rows_by_run = !out_depth && b->opts.min_parent && b->out_depth;
     if (stop) { BD_CUDA(cudaEventRecord(stop, b->stream)); }
     return BD_OK;
 }
@@ -1794,8 +1796,8 @@ bd_status collect(bd_bfs *b, bd_run_stats *stats, double ms)
     b->last = *b->head;
     b->ran = true;
     b->cleared = false;
-    // a min-parent run on a hub graph wrote the caller-order outputs itself
-    b->parents_final = b->out_depth != nullptr && b->opts.min_parent;
+    // (a min-parent run on a hub graph does, unless its rows went to the caller)
+    b->parents_final = b->rows_by_run;
     if (b->last.error) {
         b->ctrl_valid = false;
         return (bd_status)b->last.error;

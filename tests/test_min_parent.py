@@ -44,3 +44,22 @@ def test_min_parent_around_the_chunk_length(width, form):
         d = O.bfs_depth(off, adj, r)
         assert np.array_equal(ms.depths(i), d)
         assert np.array_equal(ms.parents(i), O.min_parent(off, adj, r, d))
+
+
+@pytest.mark.parametrize("order", [bd.ORDER_INSERTION, bd.ORDER_HUB])
+def test_getters_after_rows_went_to_the_caller(order):
+    """run_many_into on a min-parent handle: the getters show the last root."""
+    torch = pytest.importorskip("torch")
+    g = bd.Graph.rmat(11, 8, seed=3, order=order)
+    off, adj = g.csr()
+    n = g.num_vertices()
+    bfs = bd.HybridBFS(g, min_parent=True)
+    roots = [int(r) for r in g.pick_roots(1, 3)]
+    bfs.run(roots[2])
+    d = torch.empty((2, n), dtype=torch.int32, device="cuda")
+    p = torch.empty((2, n), dtype=torch.int64, device="cuda")
+    bfs.run_many_into(roots[:2], d.data_ptr(), p.data_ptr())
+    depth = O.bfs_depth(off, adj, roots[1])
+    assert np.array_equal(d[1].cpu().numpy(), depth)
+    assert np.array_equal(bfs.depths(), depth)
+    assert O.check(off, adj, roots[1], bfs.parents())
