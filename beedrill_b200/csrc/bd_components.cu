@@ -91,15 +91,16 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long x)
 //
 // The loads go through L1 (ld.ca), which is not coherent between SMs, so a
 // load may return an older value of a parent word.  That is safe: every
-// value a parent word ever holds is an ancestor of its vertex with a
+// value a parent word holds while joins run is an ancestor of its vertex with a
 // smaller id (links and path splitting only write ancestors, and a tree
 // only grows), so a stale walk still descends strictly and ends at a
 // vertex that is, or was, a root of x's tree.  A join acts on such a root
-// only through atomicCAS, which sees the current word.  What L1 buys: after
-// a sampling round nearly every vertex points at the largest tree's root,
-// and checking that root's own word from every thread put millions of
-// loads on one L2 slice (a second sampling round ran 3x slower than the
-// first); from L1 each SM loads it once.
+// only through atomicCAS, which sees the current word.  (cc_merge_kernel may
+// move a root from one tree to another, but in launches of its own, and L1
+// starts empty in each launch.)  What L1 buys: nearly every vertex points at the
+// largest tree's root by then, and checking that root's own word from every
+// thread put millions of loads on one L2 slice (three times the time of a pass
+// over the same bytes); from L1 each SM loads it once.
 __device__ __forceinline__ uint32_t cc_find(uint32_t *parent, uint32_t x)
 {
     uint32_t p = __ldca(&parent[x]);
