@@ -16,7 +16,7 @@ CU_SRCS := $(CSRC)/bd_common.cu $(CSRC)/bd_graph.cu $(CSRC)/bd_bfs.cu $(CSRC)/bd
            $(CSRC)/bd_check.cu $(CSRC)/bd_components.cu
 CU_OBJS := $(patsubst $(CSRC)/%.cu,beedrill_b200/_build/%.o,$(CU_SRCS))
 HDRS := include/beedrill_b200.h $(CSRC)/bd_internal.h $(CSRC)/bd_bfs_device.cuh $(CSRC)/bd_device_util.cuh \
-        $(CSRC)/bd_policy.cuh
+        $(CSRC)/bd_policy.cuh $(CSRC)/bd_split.h
 LIB := beedrill_b200/lib/libbeedrill_b200.so
 CLI := beedrill_b200/bin/hybrid_bfs
 CC_CLI := beedrill_b200/bin/components

@@ -287,7 +287,7 @@ __device__ void td_step(const BfsParams &p, const StepView &sv, const Team &team
     if (nch > 0) {
         // (x counts parts of chunks where there are too few chunks for the warps)
         const int cut = split_chunks(nch, p.chunk, nw);
-        const int64_t part = ((int64_t)(p.chunk >> cut) + 31) / 32 * 32;
+        const int64_t part = split_part(p.chunk, cut);
         const long long per = ((nch << cut) + nw - 1) / nw;
         const long long x0 = gw * per, x1 = min(nch << cut, x0 + per);
         const long long c0 = x0 >> cut;

@@ -3,6 +3,8 @@
 
 #include <stdint.h>
 
+#include "bd_split.h"
+
 namespace bd {
 namespace dev {
 
@@ -85,30 +87,6 @@ __device__ __forceinline__ unsigned long long warp_excl_or(unsigned long long x)
     }
     unsigned long long excl = __shfl_up_sync(kFullMask, incl, 1);
     return lane == 0 ? 0ull : excl;
-}
-
-// How finely a frontier is dealt to nw warps when it is too small to give each a
-// full round of arcs.  A warp's round costs time in proportion to its arcs (each
-// takes some eight scattered requests through the warp's SM: 128 arcs of a batched
-// push 8,000 to 12,000 cycles), so few arcs are spread thinner, down to 32
-// a warp: the first push of 64 roots 25 -> 13 us at scales 12 to 22, pushes on a
-// 509 x 523 grid 13.0 -> 9.7 ms (a quarter as many work items: 11.2).
-//
-// log2 of the parts a chunk of `chunk` arcs is cut into, of 32 arcs or more each.
-__device__ __forceinline__ int split_chunks(long long chunks, uint32_t chunk, long long nw)
-{
-    int k = 0;
-    while ((chunks << (k + 1)) <= nw && (chunk >> (k + 1)) >= 32) { ++k; }
-    return k;
-}
-
-// log2 of the vertices a warp takes at once: 32, or fewer of about 32 arcs
-// together (avg: the frontier's average degree).
-__device__ __forceinline__ int split_group(long long vertices, int avg, long long nw)
-{
-    int k = 5;
-    while (k > 0 && (avg << k) > 32 && (vertices >> (k - 1)) < nw) { --k; }
-    return k;
 }
 
 // The average degree of a frontier, at most 64 (in float: the quotient is only a

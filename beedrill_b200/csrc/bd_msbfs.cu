@@ -448,7 +448,7 @@ __device__ void ms_push_step(const MsParams &p, const MsView &sv, MsWarpScratch 
     const int new_level = sv.level + 1;
     // large frontier vertices: part of chunk c of vertex ql[i]
     const int cut = split_chunks(sv.f_chunks, p.chunk, nw);
-    const int64_t part = ((int64_t)(p.chunk >> cut) + 31) / 32 * 32;
+    const int64_t part = split_part(p.chunk, cut);
     for (long long x = gw; x < sv.f_chunks << cut; x += nw) {
         const long long c = x >> cut;
         long long lo = 0, hi = sv.f_large - 1;
