@@ -1886,13 +1886,13 @@ void bfs_free(bd_bfs *b)
 
 }  // namespace
 
-cudaError_t min_parent_alloc(const bd_graph *g, MinParentScratch *s)
+cudaError_t min_parent_alloc(const bd_graph *g, MinParentScratch *s, cudaStream_t stream)
 {
     if (g->max_degree <= kMinLong) { return cudaSuccess; }  // nothing is ever listed
     // a list of more than kMinLong arcs has less than 2 arcs / kMinLong chunks
     cudaError_t e = cudaMalloc(&s->chunks, sizeof(uint2) * (2 * g->arcs / kMinLong));
     if (e == cudaSuccess) { e = cudaMalloc(&s->count, sizeof(unsigned long long) * 2); }
-    if (e == cudaSuccess) { e = cudaMemset(s->count, 0, sizeof(unsigned long long) * 2); }
+    if (e == cudaSuccess) { e = cudaMemsetAsync(s->count, 0, sizeof(unsigned long long) * 2, stream); }
     return e;
 }
 
@@ -1967,7 +1967,7 @@ bd_status bd_bfs_create(bd_graph *g, const bd_bfs_opts *opts, bd_bfs **out)
               cudaMalloc(&b->ctrl, sizeof(Ctrl)) == cudaSuccess &&
               cudaHostAlloc(&b->head, sizeof(CtrlHead), cudaHostAllocDefault) == cudaSuccess &&
               cudaMalloc(&b->rec, sizeof(bd_step) * kRecCap) == cudaSuccess &&
-              (!o.min_parent || min_parent_alloc(g, &b->min_scratch) == cudaSuccess);
+              (!o.min_parent || min_parent_alloc(g, &b->min_scratch, b->stream) == cudaSuccess);
     for (int i = 0; i < 2 && ok; ++i) {
         ok = cudaMalloc(&b->vis[i], sizeof(uint32_t) * words) == cudaSuccess &&
              cudaMalloc(&b->qs[i], sizeof(uint32_t) * n) == cudaSuccess &&

@@ -112,7 +112,11 @@ struct MinParentScratch {
     uint2 *chunks = nullptr;              // {vertex, chunk} of long lists
     unsigned long long *count = nullptr;  // [0] chunks listed, [1] blocks done
 };
-cudaError_t min_parent_alloc(const bd_graph *g, MinParentScratch *s);
+// stream: the one the launches will be queued on; the counters are cleared in its
+// order (handles' streams do not wait for the default stream, so a clear left there
+// could come after the first launch, which would index chunks by what the memory
+// held before).
+cudaError_t min_parent_alloc(const bd_graph *g, MinParentScratch *s, cudaStream_t stream);
 void min_parent_free(MinParentScratch *s);
 // For every vertex of depth d > 0, the smallest neighbour of depth d - 1 in the
 // caller's CSR, written to parent (which holds some such neighbour already in

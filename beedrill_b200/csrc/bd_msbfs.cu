@@ -1839,7 +1839,8 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
               cudaMalloc(&b->rec, sizeof(bd_step) * kMsRecCap) == cudaSuccess &&
               cudaMalloc(&b->d_sources, sizeof(int64_t) * 64 * b->groups) == cudaSuccess &&
               cudaMalloc(&b->d_counts, sizeof(unsigned long long) * 128 * b->groups) == cudaSuccess;
-    ok = ok && (!o.min_parent || min_parent_alloc(g, &b->min_scratch) == cudaSuccess);
+    ok = ok &&
+         (!o.min_parent || min_parent_alloc(g, &b->min_scratch, b->stream) == cudaSuccess);
     for (int i = 0; i < 3 && ok; ++i) {
         ok = cudaMalloc(&b->F[i], sizeof(ull) * n) == cudaSuccess &&
              cudaMalloc(&b->qs[i], sizeof(uint32_t) * n) == cudaSuccess &&

@@ -63,3 +63,22 @@ def test_getters_after_rows_went_to_the_caller(order):
     assert np.array_equal(d[1].cpu().numpy(), depth)
     assert np.array_equal(bfs.depths(), depth)
     assert O.check(off, adj, roots[1], bfs.parents())
+
+
+def test_new_handles_beside_work_on_the_default_stream():
+    """A handle made and used while the default stream is busy, which handles'
+    streams do not wait for: its counters are clear before its first launch, and
+    nothing of its making is left to come after it."""
+    torch = pytest.importorskip("torch")
+    n, src, dst, root = _two_hubs(5000)
+    g = bd.Graph.from_edges(n, src, dst)
+    off, adj = g.csr()
+    want = O.min_parent(off, adj, root, O.bfs_depth(off, adj, root))
+    for make in (lambda: bd.HybridBFS(g, min_parent=True), lambda: bd.BatchedBFS(g, 2, min_parent=True)):
+        torch.cuda._sleep(1 << 28)  # some 0.15 s
+        handle = make()
+        parents = handle.parents if isinstance(handle, bd.HybridBFS) else lambda: handle.parents(0)
+        for _ in range(2):
+            handle.run(root if isinstance(handle, bd.HybridBFS) else [root, root])
+            assert np.array_equal(parents(), want)
+            torch.cuda.synchronize()
