@@ -1663,6 +1663,7 @@ struct bd_bfs {
     bool ran = false;
     bool parents_final = false;  // caller-visible depths and parents are up to date
     bool rows_by_run = false;    // the last run queued wrote out_depth and out_parent itself
+    bool min_due = false;        // its smallest-parent pass went over the caller's rows only
     int64_t last_source = -1;
     CtrlHead last{};
 };
@@ -1779,6 +1780,7 @@ bd_status enqueue_bfs(bd_bfs *b, int64_t count, int64_t source, cudaEvent_t star
         BD_CUDA(launch_min_parent(b->g, b->min_scratch, depth, parent, b->stream));
     }
     b->rows_by_run = !out_depth && b->opts.min_parent && b->out_depth;
+    b->min_due = out_depth && b->opts.min_parent;
     if (stop) { BD_CUDA(cudaEventRecord(stop, b->stream)); }
     return BD_OK;
 }
@@ -1836,8 +1838,8 @@ bd_status run_sources(bd_bfs *b, const int64_t *sources, int64_t count, bd_run_s
 }
 
 // Makes the caller-visible depths and parents current (queued on the handle's
-// stream): the reference's -deg / -1 encoding of unreached vertices, and on a hub graph the mapping
-// back to the caller's numbering.
+// stream): the reference's -deg / -1 encoding of unreached vertices, on a hub graph the mapping
+// back to the caller's numbering, and the smallest parents where the run left them to do.
 bd_status finalize_parents(bd_bfs *b)
 {
     if (!b->ran) { return BD_ERR_STATE; }
@@ -1850,6 +1852,10 @@ bd_status finalize_parents(bd_bfs *b)
                                                                   b->parent);
     }
     BD_CUDA(cudaGetLastError());
+    if (b->min_due) {
+        BD_CUDA(launch_min_parent(b->g, b->min_scratch, b->out_depth ? b->out_depth : b->depth,
+                                  b->out_parent ? b->out_parent : b->parent, b->stream));
+    }
     b->parents_final = true;  // in stream order
     return BD_OK;
 }

@@ -65,6 +65,33 @@ def test_getters_after_rows_went_to_the_caller(order):
     assert O.check(off, adj, roots[1], bfs.parents())
 
 
+@pytest.mark.parametrize("form", ["edges", "hub", "csr"])
+def test_getters_and_rows_hold_the_same_tree(form):
+    """run_many_into on a min-parent handle leaves the smallest parents to the
+    getters too, whatever kind of run came before or comes next."""
+    torch = pytest.importorskip("torch")
+    g = bd.Graph.rmat(12, 16, seed=7, order=bd.ORDER_HUB if form == "hub" else bd.ORDER_INSERTION)
+    off, adj = g.csr()
+    if form == "csr":
+        g = bd.Graph.from_csr(off, adj)
+    n = g.num_vertices()
+    bfs = bd.HybridBFS(g, min_parent=True)
+    roots = [int(r) for r in g.pick_roots(1, 4)]
+    want = [O.min_parent(off, adj, r, O.bfs_depth(off, adj, r)) for r in roots]
+    d = torch.empty((2, n), dtype=torch.int32, device="cuda")
+    p = torch.empty((2, n), dtype=torch.int64, device="cuda")
+    for k in (0, 2):
+        bfs.run_many_into(roots[k:k + 2], d.data_ptr(), p.data_ptr())
+        assert np.array_equal(p.cpu().numpy(), want[k:k + 2])
+        for _ in range(2):
+            assert np.array_equal(bfs.parents(), want[k + 1])
+        assert bfs.check(roots[k + 1])
+        bfs.run(roots[k])
+        assert np.array_equal(bfs.parents(), want[k])
+    bfs.run_many(roots)
+    assert np.array_equal(bfs.parents(), want[3])
+
+
 def test_new_handles_beside_work_on_the_default_stream():
     """A handle made and used while the default stream is busy, which handles'
     streams do not wait for: its counters are clear before its first launch, and
