@@ -639,10 +639,14 @@ class BatchedBFS:
 
     def counts(self):
         """(m_c, n_c) arrays over the roots of the last run."""
-        m = np.empty(self.count, np.int64)
-        n = np.empty(self.count, np.int64)
+        # The library writes one entry per root of its last run, which is another
+        # than this object's when a run has ended with a timeout since: there is
+        # room for any run's, and fewer roots than this object's is an error.
+        m = np.empty(self.max_roots, np.int64)
+        n = np.empty(self.max_roots, np.int64)
+        _check(lib().bd_msbfs_count_traversed_edges(self._h, self.count - 1, None, None), "count")
         _check(lib().bd_msbfs_counts(self._h, _ptr(m, c_int64), _ptr(n, c_int64)), "count")
-        return m, n
+        return m[:self.count], n[:self.count]
 
     def steps(self) -> list[dict]:
         count = c_int64()

@@ -316,7 +316,9 @@ bd_status bd_msbfs_get_parents(bd_msbfs *b, int32_t root_index, int64_t *parent)
 /* count_num_traversed_edges() (m_c) and reached vertices (n_c) of one root. */
 bd_status bd_msbfs_count_traversed_edges(bd_msbfs *b, int32_t root_index, int64_t *edges,
                                          int64_t *reached);
-/* The same of every root of the last run, in its order (either may be NULL). */
+/* The same of every root of the last run, in its order (either may be NULL).  A run
+   that ended with BD_ERR_TIMEOUT counts as the last one: arrays of max_roots entries
+   have room for any. */
 bd_status bd_msbfs_counts(bd_msbfs *b, int64_t *edges, int64_t *reached);
 /* hybrid_bfs::check (hybrid_bfs.cc:281-379) of one root's parents. */
 bd_status bd_msbfs_check(bd_msbfs *b, int32_t root_index, int32_t *ok);
