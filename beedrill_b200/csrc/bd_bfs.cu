@@ -832,6 +832,9 @@ __device__ __forceinline__ void record_step(const BfsParams &p, const LevelState
 // Grid barrier number b: arrival (one release-add) and polling until every CTA
 // has arrived, at most p.spin_limit polls; running out sets
 // ctrl->error = BD_ERR_TIMEOUT.  Thread 0 of each CTA.  False after an error.
+// solo: CTA 0 arrives only after levels of its own, or a long list of sources;
+// the bound then holds for each of these (p.spin_limit polls in which ctrl->beat
+// does not change), as it does for a level of the grid.
 __device__ __forceinline__ bool arrive_wait(const BfsParams &p, long long b, bool solo)
 {
     Ctrl *c = p.ctrl;
@@ -843,10 +846,16 @@ __device__ __forceinline__ bool arrive_wait(const BfsParams &p, long long b, boo
     // among them, then went to L2: 4.1 us a level instead of 2.6).  At the end of
     // a grid step the waits are short, and a poll that is itself the acquire
     // saves a round trip (0.4 us a level).
+    unsigned long long beat = solo ? ld_relaxed64(&c->beat) : 0ull;
     while (solo && ld_relaxed64(&c->bar) < target) {
         if (++it > p.spin_limit) {
-            atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
-            return false;
+            const unsigned long long now = ld_relaxed64(&c->beat);
+            if (now == beat) {
+                atomicExch(&c->error, (int)BD_ERR_TIMEOUT);
+                return false;
+            }
+            beat = now;
+            it = 0;
         }
         __nanosleep(64);
     }
@@ -1139,6 +1148,7 @@ __device__ void solo_init(const BfsParams &p, SharedState<BLOCK> &sh, SoloQueues
                           Local &loc)
 {
     for (int64_t i0 = (int64_t)(threadIdx.x & ~31u); i0 < p.source_count; i0 += BLOCK) {
+        if (threadIdx.x == 0 && i0) { st_relaxed64(&p.ctrl->beat, globaltimer()); }
         const int64_t i = i0 + lane_id();
         bool has[1] = {i < p.source_count};
         uint32_t v[1] = {0u};
@@ -1229,6 +1239,7 @@ __device__ __noinline__ void solo_run(bool init)
             a.degsum = td;
             a.small_cnt = sh.acc.small_cnt;
             a.large_packed = sh.acc.large_packed;
+            st_relaxed64(&p.ctrl->beat, t_end);
             record_step(p, st, (long long)tf, t_end);
             advance(st, p, a, t_end);
             decide_rule(st, p, sh.rule_dir, sh.consult);

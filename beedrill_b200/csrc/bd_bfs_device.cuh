@@ -83,6 +83,7 @@ struct alignas(16) CtrlHead {
 struct Ctrl : CtrlHead {
     LevelState pub[2];           // published by CTA 0 at barrier b, in slot b % 2
     Acc acc[3];
+    unsigned long long beat;     // changes while CTA 0 works alone: its last level's time
 };
 
 struct BfsParams {

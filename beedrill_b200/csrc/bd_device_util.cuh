@@ -25,6 +25,11 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
     return v;
 }
 
+__device__ __forceinline__ void st_relaxed64(unsigned long long *p, unsigned long long v)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 // Arrival at a grid barrier: orders every write the CTA made before it (the
 // CTA synchronised with __syncthreads first) ahead of the increment.
 __device__ __forceinline__ void red_release_add64(unsigned long long *p, unsigned long long v)

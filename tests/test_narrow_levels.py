@@ -92,6 +92,19 @@ def test_many_sources(order, count):
     assert np.array_equal(parent[want == 0], np.flatnonzero(want == 0))
 
 
+def test_long_source_lists_under_a_short_wait_bound():
+    """spin_limit bounds the wait for one level.  CTA 0 needs several times as long
+    for the sources (2048 rounds of some 3 us, against 2000 polls of about 0.7 us);
+    the levels themselves, and the whole call before sources were set up by the one
+    launch, stay far below it."""
+    g = bd.Graph.rmat(20, 8, seed=1)
+    n = g.num_vertices()
+    bfs = bd.HybridBFS(g, spin_limit=2000)
+    assert bfs.run_multi(np.arange(n)).reached == n
+    assert not bfs.depths().any()
+    assert np.array_equal(bfs.parents(), np.arange(n))
+
+
 @pytest.mark.parametrize("scale", [8, 11, 12, 13])
 def test_small_graphs_bottom_up(scale):
     g = bd.Graph.rmat(scale, 6, seed=scale)
