@@ -1906,11 +1906,7 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
             4096, std::max<int64_t>(32, per_warp < 65536 ? per_warp / 80 : per_warp / 32));
         if (!g->d_perm && g->max_degree <= 1024) { b->opts.heavy_degree = 1024; }
     }
-    // chunks of about two such lengths (scale 22, heavy_degree 512: 4.59 with 512
-    // arcs, 4.63 with 2048)
-    if (b->opts.heavy_chunk <= 0) {
-        b->opts.heavy_chunk = std::min(2048, std::max(128, 2 * b->opts.heavy_degree));
-    }
+    if (b->opts.heavy_chunk <= 0) { b->opts.heavy_chunk = dev::long_chunk(b->opts.heavy_degree); }
     b->opts.pull_prefix = std::min(b->opts.pull_prefix, b->opts.heavy_degree);
     // room for every chunk a pull step can leave to ms_pull_long
     {

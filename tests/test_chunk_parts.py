@@ -15,6 +15,7 @@ extern "C" int cut_of(long long chunks, unsigned chunk, long long nw)
 {
     return bd::dev::split_chunks(chunks, chunk, nw);
 }
+extern "C" int long_chunk(int arcs) { return bd::dev::long_chunk(arcs); }
 extern "C" long long part_of(unsigned chunk, int cut) { return bd::dev::split_part(chunk, cut); }
 """
 
@@ -37,6 +38,11 @@ def test_parts_cover_their_chunk(split):
         for cut in range(split.cut_of(1, chunk, 1 << 40) + 1):
             part = split.part_of(chunk, cut)
             assert part % 32 == 0 and part << cut >= chunk, (chunk, cut, part)
+
+
+def test_chunks_of_long_lists_for_any_heavy_degree(split):
+    for arcs in (1, 63, 64, 65, 1023, 1024, 1025, 4096, 2**30 - 1, 2**30, 2**31 - 1):
+        assert split.long_chunk(arcs) == min(2048, max(128, 2 * arcs)), arcs
 
 
 def _star(leaves):
