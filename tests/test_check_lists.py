@@ -1,6 +1,8 @@
 """The device check around the list lengths at which it changes who looks through
 a list (16 and 2048 arcs) or splits it (1024), on symmetric graphs and on a
 caller's CSR, with a tree that is right and with one mistake."""
+import time
+
 import numpy as np
 import pytest
 
@@ -41,3 +43,22 @@ def test_long_lists(width, form):
     for r in (root, last, odd):
         bfs.run(r)
         assert bfs.check(r) and bfs.check(r)
+
+
+def test_a_small_graph_takes_no_longer_than_a_large_one():
+    """A frontier of a few vertices with lists of hundreds of arcs is dealt to many
+    warps: as one warp's work it made the check of a scale-14 graph three times as
+    long as that of a graph 16 times its size (the bound allows 1.5 times)."""
+    best = {}
+    for scale in (14, 18):
+        g = bd.Graph.rmat(scale, 16, seed=scale, order=bd.ORDER_HUB)
+        root = int(g.pick_roots(3, 8)[7])
+        bfs = bd.HybridBFS(g)
+        bfs.run(root)
+        times = []
+        for _ in range(16):
+            t0 = time.perf_counter()
+            assert bfs.check(root)
+            times.append(time.perf_counter() - t0)
+        best[scale] = min(times)
+    assert best[14] < 1.5 * best[18], best
