@@ -224,17 +224,60 @@ __global__ void __launch_bounds__(kMergeThreads) cc_merge_kernel(const uint32_t 
 }
 
 // Every vertex pointed at its root (a vertex already there is not
-// written).  No join runs meanwhile, so the roots are fixed; the walks do
-// not split paths, so no thread moves a word another thread has already
-// pointed at its root.
-__global__ void cc_flatten_kernel(uint32_t *parent, int64_t n, const uint32_t *wanted)
+// written).  No join runs meanwhile, so the roots are fixed, and a thread
+// writes its own vertex's word only, so none moves a word that has already
+// been pointed at its root.  A walk longer than kNear moves that word along as
+// it goes, and reads past L1: walks that come through the vertex then jump as
+// far as its own has come, and a chain is crossed in some log2 of its length.
+// (Hooking makes chains wherever ids follow a path, as in the rows of a grid.)
+// Blocks start in the order of the ids, each with the next F * kThreads, and
+// chains lead to smaller ids, so that they end where a block has been: a
+// 4000 x 4003 grid took 1750 us in blocks that stride over the ids, without
+// moving words, and takes 210.
+constexpr int kNear = 8;
+template <int F>
+__global__ void __launch_bounds__(kThreads) cc_flatten_kernel(uint32_t *parent, int64_t n,
+                                                              const uint32_t *wanted)
 {
     if (wanted && *wanted == 0) { return; }
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t p = __ldcg(&parent[v]);
-        const uint32_t r = cc_root(parent, p);
-        if (r != p) { __stcg(&parent[v], r); }
+    const int64_t first = blockIdx.x * (int64_t)(F * kThreads) + threadIdx.x;
+    uint32_t p[F], up[F];
+#pragma unroll
+    for (int k = 0; k < F; ++k) {
+        const int64_t v = first + k * kThreads;
+        p[k] = v < n ? __ldcg(&parent[v]) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < F; ++k) { up[k] = __ldca(&parent[p[k]]); }
+#pragma unroll
+    for (int k = 0; k < F; ++k) {
+        const int64_t v = first + k * kThreads;
+        if (v >= n || up[k] == p[k]) { continue; }
+        uint32_t r = up[k], q = __ldca(&parent[r]);
+        for (int i = 1; i < kNear && q != r; ++i) {
+            r = q;
+            q = __ldca(&parent[r]);
+        }
+        while (q != r) {
+            __stcg(&parent[v], q);
+            r = q;
+            q = __ldcg(&parent[r]);
+        }
+        __stcg(&parent[v], r);
+    }
+}
+
+// Two vertices a thread where five device-fuls of threads and more have a vertex
+// each (148 SMs x 2048 threads): fewer blocks, and the reads of two walks at once.  A run
+// in us with one and with two: grid 1021 x 1031 110, 134; 1400 x 1402 151, 140; scale
+// 22 225, 203; 24 735, 649.
+void launch_flatten(uint32_t *parent, int64_t n, const uint32_t *wanted, cudaStream_t s)
+{
+    const int64_t blocks = std::max<int64_t>(1, (n + kThreads - 1) / kThreads);
+    if (n < 5ll * 148 * 2048) {
+        cc_flatten_kernel<1><<<(unsigned)blocks, kThreads, 0, s>>>(parent, n, wanted);
+    } else {
+        cc_flatten_kernel<2><<<(unsigned)((blocks + 1) / 2), kThreads, 0, s>>>(parent, n, wanted);
     }
 }
 
@@ -553,12 +596,12 @@ bd_status bd_components_run(bd_components *c, bd_components_stats *stats)
         uint32_t *second = reinterpret_cast<uint32_t *>(c->label);
         bd::cc_hook_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(g->d_off, g->d_adj, n, c->parent,
                                                                     second, c->size);
-        bd::cc_flatten_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, nullptr);
+        bd::launch_flatten(c->parent, n, nullptr, s);
         const int merge_grid = std::min(bd::grid_for(n) / 4 + 1, 148 * 2);
         const uint32_t *wanted = nullptr;  // the last round's kernels ask the probe
         for (int round = 0; round <= bd::kMergeRounds; ++round) {
             bd::cc_merge_kernel<<<merge_grid, bd::kMergeThreads, 0, s>>>(second, n, c->parent, wanted);
-            bd::cc_flatten_kernel<<<bd::grid_for(n), bd::kThreads, 0, s>>>(c->parent, n, wanted);
+            bd::launch_flatten(c->parent, n, wanted, s);
             if (round + 1 >= bd::kMergeRounds) {
                 bd::cc_probe_kernel<<<1, bd::kProbe, 0, s>>>(c->parent, n, g->d_isolated, c->giant,
                                                              wanted);

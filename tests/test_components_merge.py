@@ -45,3 +45,46 @@ def test_ragged_pieces(pieces, form):
         assert np.array_equal(c.labels(), labels)
         assert np.array_equal(c.sizes(), sizes)
         assert c.check()
+
+
+def _comb(spine, teeth):
+    """A path of `spine` vertices, a path of `teeth` more hanging from each."""
+    v = np.arange(spine - 1)
+    src, dst, prev = [v], [v + 1], np.arange(spine)
+    for k in range(1, teeth + 1):
+        cur = k * spine + np.arange(spine)
+        src.append(prev)
+        dst.append(cur)
+        prev = cur
+    return spine * (teeth + 1), np.concatenate(src), np.concatenate(dst)
+
+
+def test_ids_along_a_path_take_no_longer_than_shuffled_ones():
+    """Chains of parents as long as the graph is deep, which hooking makes of ids
+    that follow a path, are crossed in steps that double.  Walked arc by arc they
+    made this comb three times as slow as the same one with shuffled ids."""
+    n, src, dst = _comb(100000, 3)
+    ids = np.random.default_rng(0).permutation(n)
+    best = []
+    for s, d in ((src, dst), (ids[src], ids[dst])):
+        c = bd.Components(bd.Graph.from_edges(n, s, d))
+        assert c.run().num_components == 1
+        best.append(min(c.run().ms for _ in range(9)))
+    assert best[0] < 1.5 * best[1], best
+
+
+@pytest.mark.parametrize("n", [5 * 148 * 2048 + d for d in (-257, -1, 0, 1, 255, 256, 257)])
+def test_chains_around_the_flattening_s_border(n):
+    """Ids along two paths with an isolated vertex between, at sizes around the one
+    from which a thread points two vertices at their roots."""
+    half = n // 2
+    v = np.concatenate([np.arange(half - 1), np.arange(half + 1, n - 1)])
+    c = bd.Components(bd.Graph.from_edges(n, v, v + 1))
+    for _ in range(2):
+        assert c.run().num_components == 3
+    want = np.zeros(n, np.int64)
+    want[half:] = half + 1
+    want[half] = half
+    assert np.array_equal(c.labels(), want)
+    sizes = c.sizes()
+    assert (sizes[0], sizes[half], sizes[half + 1]) == (half, 1, n - half - 1)
