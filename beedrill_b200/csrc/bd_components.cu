@@ -59,6 +59,7 @@
 
 #include <algorithm>
 
+#include "bd_device_util.cuh"
 #include "bd_internal.h"
 
 namespace bd {
@@ -70,6 +71,7 @@ constexpr int64_t kHeavy = 4096;    // arcs above which a vertex is split over t
 constexpr int kHookArcs = 4;        // arcs a vertex looks at for its first parent
 constexpr int kMergeRounds = 2;     // and a third where the probe asks for it
 constexpr int kProbeOutside = 4;    // probed vertices outside the largest tree that do
+constexpr int kProbeInside = 2;     // ... unless it holds no two of them
 constexpr int kProbe = 256;         // vertices whose roots vote for the largest tree (one block)
 constexpr int64_t kHeavyChunk = 1024;  // arcs per unit of the heavy pass
 
@@ -286,8 +288,10 @@ void launch_flatten(uint32_t *parent, int64_t n, const uint32_t *wanted, cudaStr
 // pays, because kProbeOutside of them have neighbours but lie outside that tree (a
 // second large tree is left now and then; the walk would then read all its arcs:
 // scale 22 in file order 373 us without the third round, 278 with it, where other
-// graphs lose 20 to 75 us by a round they do not need).  One block, so that the
-// host need not look.
+// graphs lose 20 to 75 us by a round they do not need) -- unless no two share a
+// root, as in a forest of small trees, where no large one is in the making (a
+// shuffled path of 3 M vertices 330 -> 280 us).  One block, so that the host need
+// not look.
 __global__ void __launch_bounds__(kProbe) cc_probe_kernel(const uint32_t *parent, int64_t n,
                                                           const uint32_t *isolated, uint32_t *giant,
                                                           const uint32_t *wanted)
@@ -317,19 +321,28 @@ __global__ void __launch_bounds__(kProbe) cc_probe_kernel(const uint32_t *parent
     const int outside = __syncthreads_count(mine != g && !lone);
     if (threadIdx.x == 0) {
         giant[0] = g;
-        giant[1] = outside >= kProbeOutside;
+        giant[1] = outside >= kProbeOutside && (unsigned)(m >> 32) >= kProbeInside;
     }
 }
 
+struct CcWalk {
+    int32_t incl[32];
+    int64_t beg[32];
+};
+
 // The arcs of the vertices of a warp's 32-vertex group that have
-// work: each such vertex's list is walked by the whole warp, 32 arcs a
-// round; lists longer than kHeavy are appended to `heavy` instead.
+// work, laid end to end and dealt to the lanes, 32 a round (list by list, a graph
+// without a large tree kept two lanes busy at degree 2: a shuffled path of 3 M
+// vertices 295 us, now 75);
+// lists longer than kHeavy are appended to `heavy` instead.
 // giant: vertices whose root is this id have no work (the largest tree); null:
 // every vertex has.
 __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
     const int64_t *off, const uint32_t *adj, int64_t n, uint32_t *parent, const uint32_t *giant,
     uint32_t *heavy, unsigned long long *heavy_count)
 {
+    __shared__ CcWalk scratch[kWarps];
+    CcWalk &ws = scratch[threadIdx.x >> 5];
     const uint32_t skip_root = giant ? *giant : 0u;
     const int lane = threadIdx.x & 31;
     const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -350,17 +363,22 @@ __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
                 work = false;
             }
         }
-        unsigned todo = __ballot_sync(0xffffffffu, work);
-        while (todo) {
-            const int owner = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int64_t bb = __shfl_sync(0xffffffffu, b, owner);
-            const int64_t ee = __shfl_sync(0xffffffffu, e, owner);
-            const uint32_t uu = (uint32_t)(base + owner);
-            for (int64_t k = bb + lane; k < ee; k += 32) {
-                cc_join(parent, uu, __ldg(&adj[k]));
+        const int32_t incl = dev::warp_incl_scan(work ? (int32_t)(e - b) : 0);
+        const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        if (total == 0) { continue; }
+        ws.incl[lane] = incl;
+        ws.beg[lane] = b;
+        __syncwarp();
+        for (int32_t k = lane; k < total; k += 32) {
+            int at = 0;  // lists that end at or before arc k
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                if (ws.incl[at + d - 1] <= k) { at += d; }
             }
+            const int64_t arc = ws.beg[at] + (k - (at ? ws.incl[at - 1] : 0));
+            cc_join(parent, (uint32_t)(base + at), __ldg(&adj[arc]));
         }
+        __syncwarp();
     }
 }
 

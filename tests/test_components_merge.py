@@ -88,3 +88,25 @@ def test_chains_around_the_flattening_s_border(n):
     assert np.array_equal(c.labels(), want)
     sizes = c.sizes()
     assert (sizes[0], sizes[half], sizes[half + 1]) == (half, 1, n - half - 1)
+
+
+@pytest.mark.parametrize("degree", [1, 2, 31, 33, 4096, 4097])
+def test_walk_over_lists_of_one_length(degree):
+    """No large tree: stars and pairs side by side, so that every list is walked,
+    those of the hubs at lengths around a warp's round and the heavy pass."""
+    stars = 3 if degree > 100 else 400
+    base = np.arange(stars) * (degree + 1)
+    src = np.repeat(base, degree)
+    dst = src + np.tile(np.arange(1, degree + 1), stars)
+    n = stars * (degree + 1)
+    ids = np.random.default_rng(degree).permutation(n)
+    for form in ("edges", "csr"):
+        g = bd.Graph.from_edges(n, ids[src], ids[dst])
+        off, adj = g.csr()
+        if form == "csr":
+            g = bd.Graph.from_csr(off, adj)
+        labels, sizes, count, _ = O.components(off, adj)
+        c = bd.Components(g)
+        assert c.run().num_components == count == stars
+        assert np.array_equal(c.labels(), labels)
+        assert np.array_equal(c.sizes(), sizes)
