@@ -236,6 +236,8 @@ template <int BLOCK>
 constexpr long long kSoloBu = 8 * BLOCK;
 template <int BLOCK>
 constexpr long long kSoloBuArcs = 64 * BLOCK;
+template <int BLOCK>
+constexpr long long kSoloBuFew = 16 * BLOCK;  // above half of kSoloBu vertices
 
 // Two queues of vertices: id, low word of the list start, and its high 16 bits
 // with the degree (65535: that or more), which becomes the position of the list's
@@ -949,7 +951,12 @@ __device__ __forceinline__ void bu_layout(const BfsParams &p, const StepView &sv
 // queues within the memory of the grid's own scratch, since a CTA that holds more
 // shared memory leaves less L1 for the bottom-up steps.  Bottom-up levels run here
 // in graphs of at most kSoloBu vertices while the lists of the unvisited ones hold
-// at most kSoloBuArcs arcs (1024 vertices: 28 -> 14 us for a whole search).
+// at most kSoloBuArcs arcs, or kSoloBuFew: the grid is better at many arcs the more
+// words there are to share, but in a hub numbering 32 vertices of the highest
+// degrees make one word and one warp's work.  Six searches bottom-up throughout in
+// ms, all steps on the grid, up to kSoloBuArcs and up to kSoloBuFew in CTA 0:
+// 1024 vertices, 16 edges each 0.67, 0.35, 0.69; 4096, 4 each 0.65, 0.77, 0.63 in
+// file order and 2.10, 0.82, 2.06 in hub order; grid 60 x 60 3.72, 3.34, 2.97.
 // Levels before CTA 0 meets the others once, so that none polls for long.
 constexpr int kSoloLevels = 128;
 
@@ -961,8 +968,9 @@ __device__ __forceinline__ bool solo_applies(const LevelState &st, const BfsPara
     if (st.dir == kDirTD) {
         return st.f_count <= kSoloCap<BLOCK> && st.f_degsum <= kSoloArcs<BLOCK>;
     }
-    return st.dir == kDirBU && p.n <= kSoloBu<BLOCK> &&
-           2 * p.m - st.visited_degsum <= kSoloBuArcs<BLOCK>;
+    const long long arcs = 2 * p.n <= kSoloBu<BLOCK> || p.perm ? kSoloBuArcs<BLOCK>
+                                                               : kSoloBuFew<BLOCK>;
+    return st.dir == kDirBU && p.n <= kSoloBu<BLOCK> && 2 * p.m - st.visited_degsum <= arcs;
 }
 
 __device__ __forceinline__ uint32_t solo_hi(int64_t beg, int64_t deg)

@@ -114,3 +114,17 @@ def test_small_graphs_bottom_up(scale):
             for root in g.pick_roots(scale, 3):
                 bfs.run(int(root))
                 _verify(bfs, g, int(root))
+
+
+@pytest.mark.parametrize("order", [bd.ORDER_INSERTION, bd.ORDER_HUB])
+@pytest.mark.parametrize("scale,factor", [(9, 30), (10, 30), (11, 4), (12, 4), (12, 16), (13, 2)])
+def test_small_graphs_bottom_up_in_either_layout(scale, factor, order):
+    """Graphs on both sides of the sizes and arc counts up to which one CTA takes a
+    bottom-up level, which depend on the numbering."""
+    g = bd.Graph.rmat(scale, factor, seed=scale + factor, order=order)
+    for block in (256, 512):
+        for alg in ("bottom_up", "beamer_hybrid"):
+            bfs = bd.HybridBFS(g, alg=alg, block_size=block)
+            for root in g.pick_roots(scale, 3):
+                bfs.run(int(root))
+                _verify(bfs, g, int(root))
