@@ -65,7 +65,6 @@ constexpr int64_t kLong = 1024;         // arcs above which a queued list is cut
 constexpr int64_t kBlockList = 2048;    // arcs above which a whole CTA looks through a list
 constexpr int kShift = 38;              // long-queue counter: vertices << 38 | chunks
 constexpr unsigned long long kLowMask = (1ull << kShift) - 1;
-constexpr long long kSpin = 4000000;    // ~2 s of polling
 using ull = unsigned long long;
 using namespace dev;
 
@@ -93,6 +92,7 @@ struct CheckParams {
     const uint32_t *adj;
     int64_t n, arcs;
     bool symmetric;
+    long long polls;  // bound of a barrier's wait
     int32_t *depth;
     uint32_t *qs[2], *ql[2];
     ull *cb[2];  // first chunk of each entry of ql
@@ -107,8 +107,8 @@ __device__ bool check_barrier(const CheckParams &p, long long b, int &flag)
         red_release_add64(&p.ctl->bar, 1ull);
         const ull target = (ull)(b + 1) * gridDim.x;
         long long it = 0;
-        while (ld_acquire64(&p.ctl->bar) < target && ++it <= kSpin) { __nanosleep(32); }
-        if (it > kSpin) { atomicExch(&p.ctl->error, (int)BD_ERR_TIMEOUT); }
+        while (ld_acquire64(&p.ctl->bar) < target && ++it <= p.polls) { __nanosleep(32); }
+        if (it > p.polls) { atomicExch(&p.ctl->error, (int)BD_ERR_TIMEOUT); }
         flag = __ldcg(&p.ctl->error);
     }
     __syncthreads();
@@ -470,6 +470,7 @@ CheckParams check_params(const bd_graph *g, const CheckScratch &s)
     p.n = g->n;
     p.arcs = g->arcs;
     p.symmetric = g->symmetric;
+    p.polls = check_polls(g->max_degree);
     p.depth = s.depth;
     for (int i = 0; i < 2; ++i) {
         p.qs[i] = s.qs[i];

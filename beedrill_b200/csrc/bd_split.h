@@ -43,6 +43,11 @@ BD_HOST_DEVICE int32_t long_chunk(int32_t arcs)
     return arcs < 64 ? 128 : arcs < 1024 ? 2 * arcs : 2048;
 }
 
+// Polls a barrier of the device check waits at most: some 2 s, and more where a list
+// is long, since one warp may look through it between two barriers, 128 arcs in the
+// time of two or three polls (the bound allows 32 such lists, a warp's share).
+BD_HOST_DEVICE long long check_polls(long long max_degree) { return 4000000 + max_degree; }
+
 // log2 of the vertices a warp takes at once: 32, or fewer of about 32 arcs
 // together (avg: the frontier's average degree).
 BD_HOST_DEVICE int split_group(long long vertices, int avg, long long nw)

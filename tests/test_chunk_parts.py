@@ -15,6 +15,7 @@ extern "C" int cut_of(long long chunks, unsigned chunk, long long nw)
 {
     return bd::dev::split_chunks(chunks, chunk, nw);
 }
+extern "C" long long check_polls(long long degree) { return bd::dev::check_polls(degree); }
 extern "C" int long_chunk(int arcs) { return bd::dev::long_chunk(arcs); }
 extern "C" long long part_of(unsigned chunk, int cut) { return bd::dev::split_part(chunk, cut); }
 """
@@ -29,6 +30,7 @@ def split(tmp_path_factory):
                     str(d / "split.cc")], check=True)
     so = ctypes.CDLL(str(d / "split.so"))
     so.cut_of.argtypes = [ctypes.c_longlong, ctypes.c_uint, ctypes.c_longlong]
+    so.check_polls.argtypes, so.check_polls.restype = [ctypes.c_longlong], ctypes.c_longlong
     so.part_of.argtypes, so.part_of.restype = [ctypes.c_uint, ctypes.c_int], ctypes.c_longlong
     return so
 
@@ -43,6 +45,12 @@ def test_parts_cover_their_chunk(split):
 def test_chunks_of_long_lists_for_any_heavy_degree(split):
     for arcs in (1, 63, 64, 65, 1023, 1024, 1025, 4096, 2**30 - 1, 2**30, 2**31 - 1):
         assert split.long_chunk(arcs) == min(2048, max(128, 2 * arcs)), arcs
+
+
+def test_the_check_waits_for_the_longest_list(split):
+    # 32 lists of 128 arcs in three polls each
+    for degree in (0, 1, 1 << 20, 1 << 28, 1 << 32, 1 << 34):
+        assert split.check_polls(degree) >= max(4000000, 32 * 3 * degree // 128)
 
 
 def _star(leaves):
