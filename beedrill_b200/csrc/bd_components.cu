@@ -331,12 +331,15 @@ struct CcWalk {
 };
 
 // The arcs of the vertices of a warp's 32-vertex group that have
-// work, laid end to end and dealt to the lanes, 32 a round (list by list, a graph
-// without a large tree kept two lanes busy at degree 2: a shuffled path of 3 M
-// vertices 295 us, now 75);
-// lists longer than kHeavy are appended to `heavy` instead.
-// giant: vertices whose root is this id have no work (the largest tree); null:
-// every vertex has.
+// work; lists longer than kHeavy are appended to `heavy` instead.
+// giant: vertices whose root is this id have no work (the largest tree), and the
+// lists of the others are laid end to end and dealt to the lanes, 32 arcs a round
+// (list by list, a graph without a large tree kept two lanes busy at degree 2: a
+// shuffled path of 3 M vertices 295 us, now 75).  null: every vertex has work, and
+// the whole warp takes one list at a time.  Nothing is joined yet then, and arcs of
+// 32 vertices at once contend for the roots of the large trees more than arcs of
+// one (RMAT scale 18 given as a CSR, us a run: end to end 250, list by list 205; 8
+// arcs a vertex 245, 178; a 1000 x 1000 grid 176, 339).
 __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
     const int64_t *off, const uint32_t *adj, int64_t n, uint32_t *parent, const uint32_t *giant,
     uint32_t *heavy, unsigned long long *heavy_count)
@@ -362,6 +365,19 @@ __global__ void __launch_bounds__(kThreads) cc_walk_kernel(
                 heavy[atomicAdd(heavy_count, 1ull)] = (uint32_t)u;
                 work = false;
             }
+        }
+        if (!giant) {
+            unsigned todo = __ballot_sync(0xffffffffu, work);
+            while (todo) {
+                const int owner = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int64_t bb = __shfl_sync(0xffffffffu, b, owner);
+                const int64_t ee = __shfl_sync(0xffffffffu, e, owner);
+                for (int64_t k = bb + lane; k < ee; k += 32) {
+                    cc_join(parent, (uint32_t)(base + owner), __ldg(&adj[k]));
+                }
+            }
+            continue;
         }
         const int32_t incl = dev::warp_incl_scan(work ? (int32_t)(e - b) : 0);
         const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
