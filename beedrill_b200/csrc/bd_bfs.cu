@@ -473,8 +473,9 @@ __device__ void bu_step(const BfsParams &p, const StepView &sv, const Team &team
                     const uint32_t l = __shfl_sync(kFull, len[k], owner);
                     // (the list's end is not read again: that read stood before every
                     // scan, 10 to 20 % of a level of few words)
-                    const int64_t e = l != kFull ? first + l
-                                                 : __ldg(&p.off[__shfl_sync(kFull, v[k], owner) + 1]);
+                    const int64_t e = l != kFull
+                                          ? first + l
+                                          : __ldg(&p.off[__shfl_sync(kFull, v[k], owner) + 1]);
                     for (int64_t base = b; base < e; base += 32) {
                         const int64_t kk = base + lane;
                         bool hit = false;
@@ -944,16 +945,19 @@ __device__ __forceinline__ void bu_layout(const BfsParams &p, const StepView &sv
 // start, so a level is a chain of three round trips (arc; visited word; claim
 // with offsets) and a few block barriers.
 //
-// Levels of a 1021 x 1031 grid by frontier size, 512 threads, whole grid against
-// one CTA: up to 64 vertices 7.4 and 3.2 us, up to 256 8.6 and 4.3 us, up to 1024
-// 9.2 and 7.9 us, above 9.4 and 13.2 us (one SM's requests then bound it).  So the
-// line lies at kSoloArcs arcs (about 640 such vertices); kSoloCap keeps the
-// queues within the memory of the grid's own scratch, since a CTA that holds more
-// shared memory leaves less L1 for the bottom-up steps.  Bottom-up levels run here
-// in graphs of at most kSoloBu vertices while the lists of the unvisited ones hold
-// at most kSoloBuArcs arcs, or kSoloBuFew: the grid is better at many arcs the more
-// words there are to share, but in a hub numbering 32 vertices of the highest
-// degrees make one word and one warp's work.  Six searches bottom-up throughout in
+// Levels of a 1021 x 1031 grid by frontier size, 512 threads, medians in us of
+// levels all on the whole grid and of levels all in one CTA: up to 16 vertices 4.9
+// and 2.8, 32 to 64 5.1 and 3.1, 100 to 160 5.2 and 4.2, 180 to 240 5.7 and 4.9, 260
+// to 319 5.8 and 5.6, 321 to 380 5.8 and 6.2, 400 to 480 5.9 and 6.8, 560 to 640 5.9
+// and 10.1 (one SM's requests then bound it).  So the line lies at kSoloCap
+// vertices, which is also what keeps the queues within the memory of the grid's own
+// scratch (a CTA that holds more shared memory leaves less L1 for the bottom-up
+// steps), and at kSoloArcs arcs.
+//
+// Bottom-up levels run here in graphs of at most kSoloBu vertices while the lists of
+// the unvisited ones hold at most kSoloBuArcs arcs, or kSoloBuFew: the grid is better
+// at many arcs the more words there are to share, but in a hub numbering 32 vertices
+// of the highest degrees make one word and one warp's work.  Six searches bottom-up throughout in
 // ms, all steps on the grid, up to kSoloBuArcs and up to kSoloBuFew in CTA 0:
 // 1024 vertices, 16 edges each 0.67, 0.35, 0.69; 4096, 4 each 0.65, 0.77, 0.63 in
 // file order and 2.10, 0.82, 2.06 in hub order; grid 60 x 60 3.72, 3.34, 2.97.

@@ -1895,11 +1895,18 @@ bd_status bd_msbfs_create(bd_graph *g, int32_t max_roots, const bd_msbfs_opts *o
     // (scale 16) and sums over four batches:
     //   scale 16 (rule 32)    32: 0.14   64: 0.15   256: 0.28   4096: 0.73
     //   scale 20 (rule 83)    64: 1.74  256: 1.83   512: 1.92   1024: 2.19
-    //   scale 22 (rule 354)  128: 4.83  256: 4.81   512: 4.82   1024: 4.97
-    //   scale 24 (rule 3430) 512: 16.98 1024: 16.87 4096: 16.69
+    //   scale 21 (rule 167)  128: 2.77  256: 2.65   512: 2.79   1024: 2.96
+    //   scale 22 (rule 337)  128: 5.48  256: 5.46   512: 5.47   1024: 5.67
+    //   scale 23 (rule 681)  256: 9.12  512: 9.07  1024: 9.17   4096: 9.42
+    //   scale 24 (rule 3430) 512: 13.60 1024: 13.44 2048: 13.52 4096: 13.57
+    // (from scale 22 on the minimum is flat, so the step of the rule between 23 and
+    // 24, at 65536 arcs a warp, costs and gains 1 %).
     // Lists up to 1024 arcs in a numbering that does not put the hubs together are
     // not left at all: a word then holds one or two of them, which take less time
-    // than the barrier (scale 12, degree order: 0.111 against 0.097 ms).
+    // than the barrier.  Four batches, none left and the rule above it: degree
+    // order, longest list 801 0.383 and 0.408 ms, 943 0.363 and 0.353, 1002 0.361 and
+    // 0.383; longer lists 1168 0.426 and 0.378, 1326 0.466 and 0.404; file order 1002
+    // 0.420 and 0.400, 1326 0.557 and 0.441.
     const int64_t per_warp = g->arcs / ((int64_t)b->grid * (b->block / 32));
     if (b->opts.heavy_degree <= 0) {
         b->opts.heavy_degree = (int32_t)std::min<int64_t>(

@@ -351,7 +351,8 @@ def bench_packed(args, w, bd, order, local):
         "e2e": {"value": head["e2e_gteps"], "unit": UNIT, "h2d_bytes_per_step": 8 * len(roots),
                 "d2h_bytes_per_step": 8,
                 "note": "public API calls per step: clear, run_multi (root upload), m_c download"},
-        "gpu_launches": args.steps * (3 + 3 * len(parts)),
+        # clear and search: of the packed graph, and of each part
+        "gpu_launches": args.steps * (2 + 2 * len(parts)),
         "clocks": clocks.summary(),
     }
     print(json.dumps(line))
@@ -455,7 +456,8 @@ def bench_components(args, w, bd, local):
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 8 * n,
                 "note": "public API per step: run, then the int64 labels copied to the host"},
         "cpu_baseline": cpu,
-        "gpu_launches": 4 * args.steps,
+        # hooks, three merges, four flattens, two probes, walk, two for heavy lists, labels
+        "gpu_launches": 14 * args.steps,
         "clocks": clocks.summary(),
     }
     print(json.dumps(line))
@@ -514,7 +516,8 @@ def bench_policy_set(args, w, bd, order, local):
                    "l2": "L2 flushed (512 MB write) before each batch", "parallelism": "1 GPU"},
         "modes": modes,
         "directions": {k: sorted(set(v)) for k, v in dirs.items()},
-        "gpu_launches": args.steps * 2 * len(graphs) * 3,
+        # clear, init, traversal and per-lane counts of each batch
+        "gpu_launches": args.steps * 2 * len(graphs) * 4,
         "clocks": clocks.summary(),
     }
     print(json.dumps(line))
@@ -820,14 +823,14 @@ def main():
                 "note": f"public API per step ({best if best in e2e_runs else 'none'}): the run "
                         "(roots uploaded by the call), m_c / n_c read back, and every root's int64 "
                         "parent array copied to pinned host memory"},
-        # kernels per root (init, traversal, result rows, counters) or per
-        # group (init, traversal, per-lane counts, result rows); the e2e
-        # passes launch the same kernels again
+        # kernels per root (clear, search with its source setup and counters, result
+        # rows) or per group (clear, init, traversal, per-lane counts, result rows);
+        # the e2e passes launch the same kernels again
         "gpu_launches": args.steps * (
-            sum({"plain": 4 * num_roots, "learned": 4 * num_roots, "plain_traversal": 3 * num_roots,
-                 "batched": 4 * groups, "batched_rule": 4 * groups,
-                 "batched_traversal": 3 * groups}[x] for x in order_run)
-            + sum({"batched": 4 * groups, "plain": 4 * num_roots}[x] for x in e2e_ways)),
+            sum({"plain": 3 * num_roots, "learned": 3 * num_roots, "plain_traversal": 2 * num_roots,
+                 "batched": 5 * groups, "batched_rule": 5 * groups,
+                 "batched_traversal": 4 * groups}[x] for x in order_run)
+            + sum({"batched": 5 * groups, "plain": 3 * num_roots}[x] for x in e2e_ways)),
         "clocks": clocks.summary(),
     }
     if el64 is not None:
